@@ -268,3 +268,13 @@ def test_default_forms_against_the_walk(eng, family, param, n0, n1, f0, f1):
 
     fast, walk = run(0), run(1)
     assert fast == walk
+
+
+@pytest.mark.parametrize("family,param", [(O.MERSENNE, 0), (O.PROTH, 3), (O.PROTH, 4), (O.RIESEL, 6),
+                                          (O.SMARANDACHE, 7), (O.SMARANDACHE, 10), (O.FIBONACCI, 0), (O.LUCAS, 0),
+                                          (O.TRIBONACCI, 0), (O.PROTH_FIXED_N, 5), (O.RIESEL_FIXED_N, 5)])
+@pytest.mark.parametrize("n0,terms", [(0, 1), (1, 255), (2, 257), (3, 1030)])
+def test_the_prime_2_alone(eng, family, param, n0, terms):
+    # one thread a term; [0, 3) holds no odd prime
+    got = run_gpu(eng, family, param, n0, n0 + terms, 0, 3, 2)
+    assert text(got) == O.trial_factor(family, param, n0, n0 + terms, 0, 3, 2, threads=1).format()
