@@ -113,7 +113,7 @@ struct ClassCounters {
     uint32_t count[CLASS_BUCKETS];  // primes per class
     uint32_t fill[CLASS_BUCKETS];   // regroup cursors
     unsigned long long next;        // walk work counter
-    uint32_t nrefine;               // primes listed for the rare-prime refinement
+    uint32_t nrefine;               // primes listed for the rare-prime refinement (for their rank: Fibonacci, Lucas)
     uint32_t nlisted[8];            // primes the screen left for classification, by divisibility pattern
     uint32_t wide;                  // a prime of the launch is 2^40 or above
     uint32_t nnine;                 // primes listed for the 9th-power character
@@ -135,6 +135,8 @@ struct ResidueScratch {
     uint32_t *nine = nullptr;    // indices of the primes for the 9th-power character
     uint64_t cap = 0;  // primes
     ClassCounters *counters = nullptr;
+    void *rank_items = nullptr;  // Fibonacci, Lucas: primes whose rank is left to take (RankItem)
+    uint32_t rank_cap = 0;
 };
 ResidueScratch *residue_scratch_create(int device, int sm_count);
 void residue_scratch_destroy(ResidueScratch *rs);

@@ -2545,6 +2545,10 @@ int prepare_residue_tables(int device, std::string &err)
     return CTD_OK;
 }
 
+}  // namespace ctd
+#include "ctd_rank.cuh"
+namespace ctd {
+
 // ----------------------------------------------------------- launchers
 template <uint32_t FAM>
 static cudaError_t launch_fam(const JobView &v, const uint64_t *d_primes, uint64_t n, int grid, int block,
@@ -2581,6 +2585,7 @@ void residue_scratch_destroy(ResidueScratch *rs)
     cudaFree(rs->listed);
     cudaFree(rs->nine);
     cudaFree(rs->counters);
+    cudaFree(rs->rank_items);
     delete rs;
 }
 
@@ -2760,6 +2765,28 @@ int launch_residues(const JobView &view, const uint64_t *d_primes, uint64_t npri
         next = &scratch->counters->next;
     }
     cudaError_t rc;
+    if (next && takes_ranks(view)) {
+        const uint32_t cap = rank_list_cap(nprimes);
+        if (cap > scratch->rank_cap) {
+            cudaFree(scratch->rank_items);
+            scratch->rank_items = nullptr;
+            scratch->rank_cap = 0;
+            if (cudaMalloc(&scratch->rank_items, (size_t)cap * sizeof(RankItem)) == cudaSuccess)
+                scratch->rank_cap = cap;
+            else  // the tiles finish their primes themselves
+                (void)cudaGetLastError();
+        }
+        const RankList list{(RankItem *)scratch->rank_items, &scratch->counters->nrefine, scratch->rank_cap};
+        rc = view.family == FIBONACCI
+                 ? launch_ranks<FIBONACCI>(view, d_primes, nprimes, scratch->sm_count, stream, scratch->counters, list)
+                 : launch_ranks<LUCAS>(view, d_primes, nprimes, scratch->sm_count, stream, scratch->counters, list);
+        if (rc != cudaSuccess) {
+            err = std::string("rank kernel launch: ") + cudaGetErrorString(rc);
+            return CTD_ERR_CUDA;
+        }
+        note_kernel_launch();
+        return CTD_OK;
+    }
     switch (view.family) {
     case MERSENNE: rc = launch_fam<MERSENNE>(view, d_primes, nprimes, grid, block, stream, next); break;
     case PROTH: rc = launch_fam<PROTH>(view, d_primes, nprimes, grid, block, stream, next); break;
