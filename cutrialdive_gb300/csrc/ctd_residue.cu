@@ -1145,12 +1145,13 @@ __device__ __forceinline__ uint64_t trib_add(uint64_t x, uint64_t y, uint64_t z,
     return addmod(addmod(x, y, p), z, p);
 }
 
-// Tribonacci: state (T(n), T(n+1), T(n+2)), two addmods per step
-// (tribonacci.hpp:566-590).  Each step computes T(n+3), which is the residue
+// The tribonacci walk for p >= 2^40, and below it under CTD_VARIANT_WALK (a
+// second algorithm for the cross-checks): state (T(n), T(n+1), T(n+2)), two
+// addmods per step.  Each step computes T(n+3), which is the residue
 // of index n+3: the first three indices are tested from the jump, then every
 // new value at its own index, so the state rotates in place (x, y, z take
 // turns holding the newest value) and the steps need no register moves.
-__device__ __forceinline__ void run_tribonacci(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
+__device__ __noinline__ void run_tribonacci_walk(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
 {
     Mont m;
     m.init(p);
@@ -1290,6 +1291,163 @@ __device__ __forceinline__ void run_tribonacci(const JobView &job, uint64_t p, u
         if (w == 0)
             push(job.fb, idx + 3 + i, p);
     }
+}
+
+// ---- tribonacci below 2^40: blocks around a centre, tested on 32-bit words
+// A block holds the exact state x0, x1, x2 = T(c), T(c+1), T(c+2) (times a
+// unit, below) and covers BACK terms before c and AHEAD after c + 2.  Each of
+// its terms is an integer combination X of x0, x1, x2, so with x_i <= p RATIO
+// a term divisible by p is X = k p with -BEHIND <= k <= MOST, and X p^-1 mod
+// 2^32 = k: the terms are generated from v_i = x_i p^-1 mod 2^32, one
+// three-input sum each, and their smallest and largest words find every zero
+// (a lane-block passes by chance once in some 200,000, settled by an exact
+// replay).  Backwards the combinations grow by 1.36 a term (1 / |the complex
+// roots|), forwards by 1.84 (the real root), so more terms are had behind the
+// centre than ahead.  The next centre is three combinations with universal
+// constants (X < 2^64) and one Montgomery reduction by 2^32 each; a common
+// factor of the state does not change its zeros, so the powers of 2^-32 are
+// left in.
+//
+// Bound by the multiply pipe and the ALU: 54 instructions a jump, of them 15
+// wide products (two slots and more each), and 2.6 a term.  Measured on the
+// 2.8 million primes of a 2^26-wide range at 2^34, n = 1..50000: 34.0 ms for
+// blocks of 18 exact 64-bit sums, 28.9 for BACK = 15 and AHEAD = 8, 26.5 for
+// the longer blocks that primes below 2^36 leave room for.  With the bounds
+// made one-sided by T(n) = 2 T(n-1) - T(n-4), which keeps an added constant,
+// the sums went to the multiply pipe (31.8 ms); blocks of 52 terms with the
+// jump's constants modulo p took 32.3.
+template <int BACK_, int AHEAD_, uint32_t BEHIND_, uint32_t MOST_>
+struct TribShape {
+    static constexpr int BACK = BACK_, AHEAD = AHEAD_, BLOCK = BACK + 3 + AHEAD;
+    static constexpr uint32_t BEHIND = BEHIND_, MOST = MOST_;
+};
+using Trib40 = TribShape<15, 8, 104, 194>;   // p < 2^40, RATIO 1 + 2^-8
+using Trib36 = TribShape<19, 9, 338, 377>;   // p < 2^36, RATIO 1 + 2^-4
+
+// T(n), T(0) = T(1) = 0, T(2) = 1
+__host__ __device__ constexpr uint32_t trib_small(int n)
+{
+    uint32_t a = 0, b = 0, c = 1;
+    for (int i = 0; i < n; ++i) {
+        const uint32_t d = a + b + c;
+        a = b, b = c, c = d;
+    }
+    return a;
+}
+
+// T(n + L) from x = T(n), y = T(n+1), z = T(n+2), times 2^-32 mod p: for x, y,
+// z <= p RATIO, at most p RATIO again
+template <int L>
+__device__ __forceinline__ uint64_t trib_jump(uint64_t x, uint64_t y, uint64_t z, uint32_t plo, uint32_t phi, uint32_t npinv)
+{
+    constexpr uint32_t cx = trib_small(L - 1), cy = trib_small(L - 1) + trib_small(L - 2), cz = trib_small(L);
+    uint64_t u = (uint64_t)(uint32_t)x * cx;
+    u += (uint64_t)(uint32_t)y * cy;
+    u += (uint64_t)(uint32_t)z * cz;
+    const uint32_t top = (uint32_t)(u >> 32) + (uint32_t)(x >> 32) * cx + (uint32_t)(y >> 32) * cy + (uint32_t)(z >> 32) * cz;
+    const uint32_t m = (uint32_t)u * npinv;
+    const uint64_t t = (uint64_t)m * plo + (uint32_t)u;  // low word 0
+    return (uint64_t)m * phi + ((t >> 32) + top);
+}
+
+// the zeros of a block by the exact recurrence; at: index of its first term
+__device__ __noinline__ void trib_replay(const JobView &job, uint64_t p, uint64_t x0, uint64_t x1, uint64_t x2,
+                                         uint64_t at, uint64_t e, int back, int ahead)
+{
+    x0 = x0 >= p ? x0 - p : x0;
+    x1 = x1 >= p ? x1 - p : x1;
+    x2 = x2 >= p ? x2 - p : x2;
+    uint64_t a = x0, b = x1, c = x2;
+#pragma unroll 1
+    for (int j = 1; j <= back; ++j) {
+        const uint64_t w = submod(submod(c, b, p), a, p), n = at + back - j;
+        c = b;
+        b = a;
+        a = w;
+        if (w == 0 && n < e)
+            push(job.fb, n - job.n0, p);
+    }
+    a = x0, b = x1, c = x2;
+#pragma unroll 1
+    for (int j = 0; j < 3 + ahead; ++j) {
+        const uint64_t n = at + back + j;
+        if (a == 0 && n < e)
+            push(job.fb, n - job.n0, p);
+        const uint64_t w = trib_add(a, b, c, p);
+        a = b;
+        b = c;
+        c = w;
+    }
+}
+
+// whether a term of the block may be a multiple of p
+template <class SHAPE>
+__device__ __forceinline__ bool trib_block(uint32_t v0, uint32_t v1, uint32_t v2)
+{
+    uint32_t t[3 + SHAPE::AHEAD];  // T(c), T(c+1), ...
+    t[0] = v0, t[1] = v1, t[2] = v2;
+#pragma unroll
+    for (int i = 3; i < 3 + SHAPE::AHEAD; ++i)
+        t[i] = t[i - 1] + t[i - 2] + t[i - 3];
+    uint32_t s[3 + SHAPE::BACK];  // T(c+2), T(c+1), T(c), T(c-1), ...
+    s[0] = v2, s[1] = v1, s[2] = v0;
+#pragma unroll
+    for (int i = 3; i < 3 + SHAPE::BACK; ++i)
+        s[i] = s[i - 3] - s[i - 2] - s[i - 1];
+    uint32_t least = __vimin3_u32(t[0], t[1], t[2]);
+#pragma unroll
+    for (int i = 3; i < 3 + SHAPE::AHEAD; i += 2)
+        least = i + 1 < 3 + SHAPE::AHEAD ? __vimin3_u32(least, t[i], t[i + 1]) : __vimin3_u32(least, t[i], s[3]);
+    uint32_t other = __vimin3_u32(s[3], s[4], s[5]), most = __vimax3_u32(s[3], s[4], s[5]);
+    static_assert(SHAPE::BACK % 2 == 1, "the terms behind go in a three and twos");
+#pragma unroll
+    for (int i = 6; i < 3 + SHAPE::BACK; i += 2) {
+        other = __vimin3_u32(other, s[i], s[i + 1]);
+        most = __vimax3_u32(most, s[i], s[i + 1]);
+    }
+    least = other < least ? other : least;
+    return (least <= SHAPE::MOST) | (most >= 0u - SHAPE::BEHIND);
+}
+
+template <class SHAPE>
+__device__ __forceinline__ void trib_walk_blocks(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
+{
+    Mont m;
+    m.init(p);
+    uint64_t x, y, z;
+    trib_triple(m, s + SHAPE::BACK, x, y, z);
+    x = m.from(x), y = m.from(y), z = m.from(z);
+    const uint32_t npinv = (uint32_t)m.pinv, pinv = 0u - npinv, plo = (uint32_t)p, phi = (uint32_t)(p >> 32);
+    // The lanes here run the blocks together, as many as the longest of them
+    // needs (terms from e on are not pushed): a vote among whichever lanes
+    // happened to be active let warps run split in two after a replay.
+    const uint32_t act = __activemask();
+    uint64_t blocks = (e - s + SHAPE::BLOCK - 1) / SHAPE::BLOCK;
+    const uint32_t high = __reduce_max_sync(act, (uint32_t)(blocks >> 32));
+    blocks = (uint64_t)high << 32 | __reduce_max_sync(act, blocks >> 32 == high ? (uint32_t)blocks : 0u);
+    for (uint64_t at = s;; at += SHAPE::BLOCK) {
+        const bool cand = trib_block<SHAPE>((uint32_t)x * pinv, (uint32_t)y * pinv, (uint32_t)z * pinv);
+        if (__any_sync(act, cand))
+            trib_replay(job, p, x, y, z, at, e, SHAPE::BACK, SHAPE::AHEAD);
+        if (--blocks == 0)
+            break;
+        const uint64_t nx = trib_jump<SHAPE::BLOCK>(x, y, z, plo, phi, npinv);
+        const uint64_t ny = trib_jump<SHAPE::BLOCK + 1>(x, y, z, plo, phi, npinv);
+        z = trib_jump<SHAPE::BLOCK + 2>(x, y, z, plo, phi, npinv);
+        x = nx, y = ny;
+    }
+}
+
+// Tribonacci (tribonacci.hpp:566-590), state (T(n), T(n+1), T(n+2)): blocks
+// below 2^40, the walk otherwise.
+__device__ __forceinline__ void run_tribonacci(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
+{
+    if (p >= (1ull << 40) || e >> 63 || job.variant == CTD_VARIANT_WALK)
+        run_tribonacci_walk(job, p, s, e);
+    else if (p >> 36)
+        trib_walk_blocks<Trib40>(job, p, s, e);
+    else
+        trib_walk_blocks<Trib36>(job, p, s, e);
 }
 
 // ----------------------------------------------------------- Smarandache

@@ -124,8 +124,9 @@ typedef struct ctd_tuning {
  * family and prime width.  WALK: the term-by-term walk (doubling families:
  * no baby-step blocks and no power-residue classes; fixed-n families: the
  * walk instead of the closed-form solve; Fibonacci/Lucas: no rank of
- * apparition; Smarandache: the 64-bit Shoup step instead of the 32-bit
- * Barrett step).  MONTGOMERY: Smarandache steps in Montgomery form (the
+ * apparition; tribonacci: one term after the other instead of blocks around
+ * a centre; Smarandache: the 64-bit Shoup step instead of the 32-bit Barrett
+ * step).  MONTGOMERY: Smarandache steps in Montgomery form (the
  * general path).  Families without such a choice ignore it. */
 #define CTD_VARIANT_AUTO 0
 #define CTD_VARIANT_WALK 1
