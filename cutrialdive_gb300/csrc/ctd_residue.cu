@@ -1312,7 +1312,8 @@ __device__ __noinline__ void run_tribonacci_walk(const JobView &job, uint64_t p,
 // wide products (two slots and more each), and 2.6 a term.  Measured on the
 // 2.8 million primes of a 2^26-wide range at 2^34, n = 1..50000: 34.0 ms for
 // blocks of 18 exact 64-bit sums, 28.9 for BACK = 15 and AHEAD = 8, 26.5 for
-// the longer blocks that primes below 2^36 leave room for.  With the bounds
+// the longer blocks that primes below 2^36 leave room for, and 23.4 with the
+// loop in a function of its own and the replay out of it.  With the bounds
 // made one-sided by T(n) = 2 T(n-1) - T(n-4), which keeps an added constant,
 // the sums went to the multiply pipe (31.8 ms); blocks of 52 terms with the
 // jump's constants modulo p took 32.3.
@@ -1410,7 +1411,7 @@ __device__ __forceinline__ bool trib_block(uint32_t v0, uint32_t v1, uint32_t v2
 }
 
 template <class SHAPE>
-__device__ __forceinline__ void trib_walk_blocks(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
+__device__ __noinline__ void trib_walk_blocks(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
 {
     Mont m;
     m.init(p);
@@ -1425,16 +1426,21 @@ __device__ __forceinline__ void trib_walk_blocks(const JobView &job, uint64_t p,
     uint64_t blocks = (e - s + SHAPE::BLOCK - 1) / SHAPE::BLOCK;
     const uint32_t high = __reduce_max_sync(act, (uint32_t)(blocks >> 32));
     blocks = (uint64_t)high << 32 | __reduce_max_sync(act, blocks >> 32 == high ? (uint32_t)blocks : 0u);
-    for (uint64_t at = s;; at += SHAPE::BLOCK) {
-        const bool cand = trib_block<SHAPE>((uint32_t)x * pinv, (uint32_t)y * pinv, (uint32_t)z * pinv);
-        if (__any_sync(act, cand))
-            trib_replay(job, p, x, y, z, at, e, SHAPE::BACK, SHAPE::AHEAD);
-        if (--blocks == 0)
-            break;
-        const uint64_t nx = trib_jump<SHAPE::BLOCK>(x, y, z, plo, phi, npinv);
-        const uint64_t ny = trib_jump<SHAPE::BLOCK + 1>(x, y, z, plo, phi, npinv);
-        z = trib_jump<SHAPE::BLOCK + 2>(x, y, z, plo, phi, npinv);
-        x = nx, y = ny;
+    // (the replay is called outside the loop over clean blocks: a call inside
+    // it cost the loop a quarter of its instructions in moves)
+    for (uint64_t at = s; blocks;) {
+        uint64_t x0, y0, z0;
+        bool hit;
+        do {
+            x0 = x, y0 = y, z0 = z;
+            hit = __any_sync(act, trib_block<SHAPE>((uint32_t)x * pinv, (uint32_t)y * pinv, (uint32_t)z * pinv));
+            x = trib_jump<SHAPE::BLOCK>(x0, y0, z0, plo, phi, npinv);
+            y = trib_jump<SHAPE::BLOCK + 1>(x0, y0, z0, plo, phi, npinv);
+            z = trib_jump<SHAPE::BLOCK + 2>(x0, y0, z0, plo, phi, npinv);
+            at += SHAPE::BLOCK;
+        } while (--blocks && !hit);
+        if (hit)
+            trib_replay(job, p, x0, y0, z0, at - SHAPE::BLOCK, e, SHAPE::BACK, SHAPE::AHEAD);
     }
 }
 
