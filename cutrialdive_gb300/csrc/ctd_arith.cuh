@@ -270,7 +270,10 @@ struct Mont32 {
             x *= 2u - p32 * x;
         pinv = (uint32_t)(0u - x);
         one = (uint64_t)(0xffffffffu % p32 + 1u) % p32;
-        r2 = one * one % p;
+        r2 = dbl(one);  // the form of 2, squared five times: of 2^32
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+            r2 = mul(r2, r2);
     }
     CTD_HD uint64_t mul(uint64_t a, uint64_t b) const
     {

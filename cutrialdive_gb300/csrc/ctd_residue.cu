@@ -1552,73 +1552,253 @@ __device__ __forceinline__ uint64_t smarandache_walk_b32(const JobView &job, uin
     return x;
 }
 
+// ---- blocks of J terms, p below 2^30 (32-bit words)
+// With x = S(m) the J terms m .. m + J - 1 of a block are the integers
+// X_i = M^i x + C_i(m), C_i(m) = sum_{l=1..i} M^(i-l) (m + l); X_i = k p with
+// 0 <= k <= 3 M^i + C_i / p <= 4 M^i for x < 3p and m + i <= p, and X_i p^-1 mod 2^32 = k.  So
+// a term's test is one multiply-add of x by p^-1 M^i, the running word
+// C_i(m) p^-1 added, and one compare, and only every J-th state is computed:
+// x(m+J) = W x + D(m), W = M^J mod p by Shoup's quotient (two of its products
+// are single-width), D(m) = C_J(m) mod p by a modular addition.  SM_GROUP
+// blocks share a vote; a group with a candidate is stepped exactly.
+//
+// Bound by integer issue (5.8 instructions a term for J = 3, 7.1 for J = 2) and
+// the multiply pipe: 4 + J slots a block (the high product takes two) where a
+// step a term took 4 a term.  Base 10, n = 10..999, the primes of a 2^26-wide
+// segment below 2^28: 1.48 ms with a step a term, 1.13 here.
+constexpr int SM_GROUP = 4;
+
+// Exact steps m -> m + 1, `count` of them, from x = S(m) < 3p: the terms
+// m .. m + count - 1 pushed where they are zeros.  Returns the last state.
+__device__ __noinline__ uint32_t smarandache_exact32(FactorsView fb, uint64_t n0, uint32_t p, uint32_t x, uint32_t M, uint32_t Ms,
+                                                     uint32_t m, uint32_t count)
+{
+#pragma unroll 1
+    for (uint32_t i = 0; i < count; ++i) {
+        if (x == 0 || x == p || x == 2 * p)
+            push(fb, (uint64_t)(m + i) - n0, p);
+        x = x * M + (m + i + 1) - mulhi32(x, Ms) * p;
+    }
+    return x;
+}
+
+// The terms m .. m + steps - 1 of one digit class (steps + m below 2^32), from
+// x = S(m) < 3p; returns S(m + steps) below 3p
+template <int J>
+__device__ __noinline__ uint32_t smarandache_blocks32(const JobView &job, Mont32 mt, uint32_t x, uint32_t M,
+                                                         uint32_t m, uint32_t steps)
+{
+    const uint32_t p = (uint32_t)mt.p, pinv = 0u - (uint32_t)mt.pinv;
+    const uint64_t Mf = mt.to(M);
+    const uint32_t Ms = mt.shoup_of_form(Mf);
+    const uint32_t groups = steps / (SM_GROUP * J);
+    if (groups) {
+        // c[i] = C_i(m) p^-1, from C_0 = 0, C_{i+1}(m) = M C_i(m) + m + i + 1;
+        // per block C_i grows by J (M^i - 1) / (M - 1)
+        uint32_t mul[J], c[J], dc[J], thr[J];
+        uint32_t power = 1, C = 0, sum = 0;  // M^i, C_i, (M^i - 1) / (M - 1) mod 2^32
+        uint64_t Wf = mt.one, Cp = 0, Sp = 0;  // M^i, C_i, (M^i - 1) / (M - 1) mod p, in Montgomery form
+        const uint64_t mf = mt.to(m);
+        uint64_t nf = mf;
+#pragma unroll
+        for (int i = 0; i < J; ++i) {
+            mul[i] = power * pinv;
+            c[i] = C * pinv;
+            dc[i] = (uint32_t)J * sum * pinv;
+            thr[i] = 4 * power + 8;  // (M^(J-1) < 2^28; the 8 for M = 0 and 1 mod p)
+            C = M * C + m + i + 1;
+            sum = M * sum + 1;
+            power *= M;
+            nf = mt.add(nf, mt.one);
+            Cp = mt.add(mt.mul(Mf, Cp), nf);
+            Sp = mt.add(mt.mul(Mf, Sp), mt.one);
+            Wf = mt.mul(Mf, Wf);
+        }
+        const uint32_t W = (uint32_t)mt.from(Wf), Ws = mt.shoup_of_form(Wf);
+        uint32_t D = (uint32_t)mt.from(Cp);
+        const uint32_t dD = (uint32_t)(mt.from(Sp) * (uint32_t)J % p);
+        // (the exact steps are called outside the loop over clean groups: a
+        // call inside it cost the loop a quarter of its instructions in moves)
+        for (uint32_t g = 0; g < groups;) {
+            uint32_t x0;
+            bool hit;
+            do {
+                x0 = x;
+                bool cand = false;
+#pragma unroll
+                for (int b = 0; b < SM_GROUP; ++b) {
+#pragma unroll
+                    for (int i = 0; i < J; ++i) {
+                        cand |= (i ? x * mul[i] + c[i] : x * pinv) < thr[i];
+                        if (i)
+                            c[i] += dc[i];
+                    }
+                    x = x * W + D - mulhi32(x, Ws) * p;
+                    D += dD;
+                    const uint32_t less = D - p;
+                    D = less < D ? less : D;  // (D < 2p: less wraps above D when D < p)
+                }
+                hit = __any_sync(__activemask(), cand);
+            } while (++g < groups && !hit);
+            if (hit)
+                smarandache_exact32(job.fb, job.n0, p, x0, M, Ms, m + (g - 1) * (SM_GROUP * J), SM_GROUP * J);
+        }
+        m += groups * (SM_GROUP * J);
+        steps -= groups * (SM_GROUP * J);
+    }
+    return smarandache_exact32(job.fb, job.n0, p, x, M, Ms, m, steps);
+}
+
+// ---- blocks of J terms, 2^30 <= p < 2^52
+// Within a digit class Y(m) = (M-1)^2 S(m) + t(m), t(m) = (M-1) m + M, obeys
+// Y(m+1) = M Y(m): p divides S(m) iff Y = t(m) (mod p) (p > M, so M - 1 is a
+// unit).  A block holds Y < 4p for its first term; term m + i is a zero only
+// if Y M^i - t(m+i) = k p with -t / p <= k < 4 M^i, and (Y M^i - t) p^-1 mod
+// 2^32 = k: one multiply-add of Y's low word and one compare a term, and only
+// every J-th Y is computed, W = M^J as an integer, Y W - q p in 64 bits:
+//   J = 2, 3: W <= 2^29 and q = mulhi(Y >> (sh-29), floor(W 2^(sh+3) / p)),
+//             within 3 of Y W / p from below (sh = floor(log2 p));
+//   J = 1:    M <= 2^20 and q = floor of a single-precision product, Y >>
+//             (sh-22) exact in 24 bits, its factor and the product rounded
+//             down: within 1.75 of Y M / p from below, so Y < 2p (a high
+//             product in its place is two more slots of the multiply pipe:
+//             5.1 against 5.5 terms a clock and SM).
+// A walk of S itself adds m in the wide product and compares with 0, p, 2p.
+// Bound by the multiply pipe (a wide product with a 64-bit sum takes nearly
+// three slots).  The primes of a 2^25-wide range at 2^34: base 10, n = 2001 ..
+// 8999 (J = 2), 4.43 ms, 6.9 with the walk of S; base 7, n = 20001 .. 24321
+// (J = 1), 4.32 and 4.50.
+__device__ __noinline__ uint64_t smarandache_exact64(FactorsView fb, uint64_t n0, uint64_t p, uint64_t Y, uint32_t M, uint64_t Ms,
+                                                     uint64_t m, uint32_t count)
+{
+    while (Y >= p)
+        Y -= p;
+    uint64_t t = ((uint64_t)(M - 1) * m + M) % p;
+#pragma unroll 1
+    for (uint32_t i = 0; i < count; ++i) {
+        if (Y == t)
+            push(fb, m + i - n0, p);
+        t = addmod(t, M - 1, p);
+        Y = Y * M - mulhi64(Y, Ms) * p;
+        Y = Y >= p ? Y - p : Y;
+    }
+    return Y;
+}
+
+// The terms m .. m + steps - 1 of one digit class from Y = Y(m) < 2p; returns
+// Y(m + steps) below p.  Ms = floor(M 2^64 / p), Ws = floor(M^J 2^64 / p).
+template <int J>
+__device__ __noinline__ uint64_t smarandache_blocks64(const JobView &job, uint64_t p, uint32_t pinv, uint64_t Y,
+                                                         uint32_t M, uint64_t Ms, uint64_t Ws, uint64_t m, uint64_t steps)
+{
+    constexpr int GROUP = J == 1 ? 8 : SM_GROUP;
+    const uint64_t groups = steps / (GROUP * J);
+    if (groups) {
+        const int sh = 63 - clz64(p);
+        const uint64_t np = (uint64_t)0 - p;
+        const uint32_t nplo = (uint32_t)np, nphi = (uint32_t)(np >> 32);
+        const uint32_t W = J == 1 ? M : J == 2 ? M * M : M * M * M;
+        const uint32_t R = (uint32_t)(Ws >> (61 - sh));
+        const float Rf = __ull2float_rd(Ws) * __int_as_float((127 - 64 + sh - 22) << 23);
+        const uint32_t below = (uint32_t)(((uint64_t)(M - 1) * (m + steps) + M) / p) + 1;
+        const uint32_t dt = (M - 1) * pinv * J;
+        uint32_t mul[J], c[J], thr[J];
+        uint32_t power = 1;
+#pragma unroll
+        for (int i = 0; i < J; ++i) {
+            mul[i] = power * pinv;
+            c[i] = below - ((M - 1) * (uint32_t)(m + i) + M) * pinv;
+            thr[i] = below + 4 * power;
+            power *= M;
+        }
+        for (uint64_t g = 0; g < groups;) {
+            uint64_t Y0;
+            bool hit;
+            do {
+                Y0 = Y;
+                bool cand = false;
+#pragma unroll
+                for (int b = 0; b < GROUP; ++b) {
+                    const uint32_t lo = (uint32_t)Y, hi = (uint32_t)(Y >> 32);
+#pragma unroll
+                    for (int i = 0; i < J; ++i) {
+                        cand |= lo * mul[i] + c[i] < thr[i];
+                        c[i] -= dt;
+                    }
+                    uint32_t q;
+                    if (J == 1)
+                        q = __float2uint_rd(__fmul_rd(__uint2float_rz(__funnelshift_r(lo, hi, sh - 22)), Rf));
+                    else
+                        q = __umulhi(__funnelshift_r(lo, hi, sh - 29), R);
+                    // lo W + q nplo in two wide products, the rest into their high
+                    // word (left to the compiler, 9 multiply-pipe instructions)
+                    asm("{\n\t.reg .b64 t;\n\t.reg .b32 a, b;\n\t"
+                        "mul.wide.u32 t, %1, %3;\n\tmov.b64 {a, b}, t;\n\tmad.lo.u32 b, %2, %3, b;\n\t"
+                        "mov.b64 t, {a, b};\n\tmad.wide.u32 t, %4, %5, t;\n\tmov.b64 {a, b}, t;\n\t"
+                        "mad.lo.u32 b, %4, %6, b;\n\tmov.b64 %0, {a, b};\n\t}"
+                        : "=l"(Y)
+                        : "r"(lo), "r"(hi), "r"(W), "r"(q), "r"(nplo), "r"(nphi));
+                }
+                hit = __any_sync(__activemask(), cand);
+            } while (++g < groups && !hit);
+            if (hit)
+                smarandache_exact64(job.fb, job.n0, p, Y0, M, Ms, m + (g - 1) * (GROUP * J), GROUP * J);
+        }
+        m += groups * (GROUP * J);
+        steps -= groups * (GROUP * J);
+    }
+    return smarandache_exact64(job.fb, job.n0, p, Y, M, Ms, m, (uint32_t)steps);
+}
+
+// Classes whose blocks take over from the walks of S: M up to 2^20 (J = 1's
+// bound) and, as going back from Y to S takes an inverse mod p (some 60
+// products, as long as 200 terms of the walk), at least this many terms unless
+// the class is the range's last; a range's last class of fewer terms than
+// SM_MIN_LAST would go by exact steps alone.
+constexpr uint64_t SM_MIN_CLASS = 2048, SM_MIN_LAST = 32;
+
 __device__ __forceinline__ void run_smarandache(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
 {
     const uint64_t b = job.param;
     uint64_t mcur = s + 1;  // m = n + 1 of the next step
     if (p < (1u << 30) && p >= e && e <= 0xffffffffull && job.variant != CTD_VARIANT_MONTGOMERY) {
-        // 32-bit Shoup path: x kept in [0, 3p) (Shoup output < 2p, plus m < p),
-        // so x = 0 mod p <=> x == p or x == 2p (x >= 1 after a step).  The
-        // set-up (the jump to Sm_b(s), the class multipliers and their Shoup
-        // quotients) in 32-bit Montgomery arithmetic: with the 64-bit form it
-        // was about 40 % of the instructions of base 10 over n = 10..1000
-        // (991 steps a prime) with every prime below 2^28
+        // 32-bit words: x kept in [0, 3p) (Shoup output < 2p, plus D < p).
+        // The set-up in 32-bit Montgomery arithmetic
         Mont32 m;
         m.init(p);
-        const uint64_t X = smarandache_at(m, b, s);
-        if (X == 0)
-            push(job.fb, s - job.n0, p);
-        const uint32_t p32 = (uint32_t)p, p2 = 2 * p32;
-        uint32_t x = (uint32_t)m.from(X);
+        uint32_t x = (uint32_t)m.from(smarandache_at(m, b, s));
         while (mcur < e) {
             uint64_t pw;
-            uint64_t cend = class_end(b, mcur, pw);
+            const uint64_t cend = class_end(b, mcur, pw);
             const uint32_t M = (uint32_t)class_multiplier(m, b, mcur, pw);
-            const uint32_t Ms = m.shoup_of_form(m.to(M));
-            uint32_t mm = (uint32_t)mcur;
-            const uint32_t mend = (uint32_t)(cend < e ? cend : e);
-            while (mm + UNROLL <= mend) {
-                const uint32_t x0 = x;
-                bool cand = false;
-#pragma unroll
-                for (int j = 0; j < UNROLL; ++j) {
-                    uint32_t q = mulhi32(x, Ms);
-                    x = x * M + (mm + j) - q * p32;
-                    cand |= (x == p32) | (x == p2);
-                }
-                if (cand) {
-                    uint32_t y = x0;
-#pragma unroll 1
-                    for (int j = 0; j < UNROLL; ++j) {
-                        uint32_t q = mulhi32(y, Ms);
-                        y = y * M + (mm + j) - q * p32;
-                        if (y == p32 || y == p2)
-                            push(job.fb, (mm + j) - job.n0, p);
-                    }
-                }
-                mm += UNROLL;
-            }
-            for (; mm < mend; ++mm) {
-                uint32_t q = mulhi32(x, Ms);
-                x = x * M + mm - q * p32;
-                if (x == p32 || x == p2)
-                    push(job.fb, mm - job.n0, p);
-            }
-            mcur = mend;
+            const uint32_t first = (uint32_t)(mcur - 1), steps = (uint32_t)((cend < e ? cend : e) - mcur);
+            // J by the chance of a candidate, 4 M^(J-1) / 2^32 a block of each
+            // lane: at M = 1000 one in 1100 for J = 3 (an eighth of a warp's
+            // groups then step exactly, and the call took 7.2 ms for the 6.1
+            // that it takes with J = 2)
+            if (M <= 128)
+                x = smarandache_blocks32<3>(job, m, x, M, first, steps);
+            else if (M <= 1u << 20)
+                x = smarandache_blocks32<2>(job, m, x, M, first, steps);
+            else
+                x = smarandache_blocks32<1>(job, m, x, M, first, steps);
+            mcur += steps;
         }
+        if (x == 0 || x == p || x == 2 * p)
+            push(job.fb, e - 1 - job.n0, p);
         return;
     }
     Mont m;
     m.init(p);
     uint64_t X = smarandache_at(m, b, s);
-    if (X == 0)
-        push(job.fb, s - job.n0, p);
     if (p < (1ull << 62) && e <= p && job.variant != CTD_VARIANT_MONTGOMERY) {
-        // 64-bit Shoup path (every m < p): x kept in [1, 3p) as r + m with
-        // r = x M - q p in [0, 2p), q = mulhi(x, floor(M 2^64 / p)); so
-        // x = 0 mod p <=> x == p or x == 2p.  The unrolled body tests the low
-        // words only; a block with a candidate is replayed with the full test.
+        // every m < p.  A class goes by blocks of Y, by the Barrett-32 walk or
+        // by the 64-bit Shoup walk; the walks keep x in [0, 3p) (x = 0 mod p
+        // <=> x in {0, p, 2p}), test the low words only and replay a block
+        // with a candidate with the full test.
         uint64_t x = m.from(X);
+        if (x == 0)
+            push(job.fb, s - job.n0, p);
         // Barrett-32 constants (p < 2^48): sh = floor(log2 p), mu = floor(2^(sh+32) / p)
         const uint32_t sh = 63 - clz64(p);
         uint32_t mu = 0;
@@ -1632,6 +1812,33 @@ __device__ __forceinline__ void run_smarandache(const JobView &job, uint64_t p, 
             const uint64_t cend = class_end(b, mcur, pw);
             const uint64_t mend = cend < e ? cend : e;
             const uint64_t M = class_multiplier(m, b, mcur, pw);
+            if (sh >= 30 && sh < 52 && pw <= (1ull << 20) && job.variant == CTD_VARIANT_AUTO &&
+                mend - mcur >= (mend == e ? SM_MIN_LAST : SM_MIN_CLASS)) {
+                // (the states x = S(m) below 3p: to() reduces them)
+                const uint64_t a = m.to(M - 1), aa = m.mul(a, a);
+                const uint64_t Yf = m.add(m.mul(aa, m.to(x)), m.add(m.mul(a, m.to(mcur - 1)), m.to(M)));
+                uint64_t Y = m.from(Yf);
+                const uint32_t pinv = 0u - (uint32_t)m.pinv;
+                const uint64_t Ms = m.shoup(M);
+                // the class's terms are mcur .. mend - 1 (mcur - 1, the state
+                // it starts from, is tested): Y goes one term ahead
+                Y = Y * M - mulhi64(Y, Ms) * p;  // < 2p
+                if (M <= 812)
+                    Y = smarandache_blocks64<3>(job, p, pinv, Y, (uint32_t)M, Ms, m.shoup(M * M * M), mcur, mend - mcur);
+                else if (M <= 23170)
+                    Y = smarandache_blocks64<2>(job, p, pinv, Y, (uint32_t)M, Ms, m.shoup(M * M), mcur, mend - mcur);
+                else
+                    Y = smarandache_blocks64<1>(job, p, pinv, Y, (uint32_t)M, Ms, Ms, mcur, mend - mcur);
+                mcur = mend;
+                if (mend < e) {
+                    // Y = Y(mend): back one term to S(mend - 1) through
+                    // Y(mend) = M ((M-1)^2 S(mend-1) + t(mend-1))
+                    const uint64_t Mf = m.to(M), tf = m.add(m.mul(a, m.to(mend - 1)), Mf);
+                    const uint64_t inv = m.pow(m.mul(aa, Mf), p - 2);
+                    x = m.from(m.mul(m.sub(m.to(Y), m.mul(Mf, tf)), inv));
+                }
+                continue;
+            }
             // Barrett-32 when 3pM + e < 2^64 and 3M + 1 <= 2^31 (x < 3p on entry either way)
             const bool b32 = mu && M < (1ull << 29) && M * 3 + 1 <= (1ull << 31) && p <= (~0ull - e) / (3 * M + 1);
             if (b32 && sh >= 32)
@@ -1646,6 +1853,8 @@ __device__ __forceinline__ void run_smarandache(const JobView &job, uint64_t p, 
         }
         return;
     }
+    if (X == 0)
+        push(job.fb, s - job.n0, p);
     // general path: Montgomery form, X' = X * (M R) + m R
     const uint64_t Rm = m.one;
     uint64_t C = m.to(mcur);

@@ -29,7 +29,7 @@ CTD_HD uint64_t class_end(uint64_t b, uint64_t m, uint64_t &pw)
 {
     pw = b;
     while (pw <= m) {
-        if (pw > ~0ull / b) {
+        if (mulhi64(pw, b)) {  // (a high product, not a division: this runs per class and prime)
             pw = ~0ull;
             return pw;
         }
