@@ -74,10 +74,12 @@ uint64_t prime_count_upper_bound(uint64_t lo, uint64_t hi);
 // Geometry of a sieve window: 16384 words of 32 odd numbers (a 2^20-wide range).
 constexpr uint64_t SIEVE_WIN_WORDS = 16384;
 constexpr uint64_t SIEVE_WIN_RANGE = 2 * 32 * SIEVE_WIN_WORDS;
+constexpr uint32_t SIEVE_WIN_CHUNKS = 4;  // chunks of a window, each with its count and offset
 constexpr uint32_t SIEVE_LEVEL0_ODD_PRIMES = 6541;  // odd primes below 2^16
 
 // Scratch for the fixed-scratch sieve (sieve_range_scratch): device pointers
-// the caller owns; bits/wcount/offsets hold `max_windows` windows.
+// the caller owns; bits/wcount/offsets hold `max_windows` windows (counts and
+// offsets: SIEVE_WIN_CHUNKS a window, and one offset more).
 struct SieveScratch {
     uint32_t *bits;
     uint32_t *wcount;

@@ -36,8 +36,8 @@ constexpr uint64_t BASE_CAP = 1100000;  // pi(2^24) = 1077871
 constexpr uint64_t align256(uint64_t x) { return (x + 255) & ~uint64_t{255}; }
 constexpr uint64_t OFF_BITS = 0;
 constexpr uint64_t OFF_WCOUNT = align256(OFF_BITS + WINDOWS * SIEVE_WIN_WORDS * 4);
-constexpr uint64_t OFF_OFFSETS = align256(OFF_WCOUNT + WINDOWS * 4);
-constexpr uint64_t OFF_BASE = align256(OFF_OFFSETS + (WINDOWS + 1) * 8);
+constexpr uint64_t OFF_OFFSETS = align256(OFF_WCOUNT + WINDOWS * SIEVE_WIN_CHUNKS * 4);
+constexpr uint64_t OFF_BASE = align256(OFF_OFFSETS + (WINDOWS * SIEVE_WIN_CHUNKS + 1) * 8);
 constexpr uint64_t OFF_LEVEL0 = align256(OFF_BASE + BASE_CAP * 4);
 constexpr uint64_t SCRATCH_BYTES = align256(OFF_LEVEL0 + 4);
 

@@ -7,13 +7,15 @@
 //
 // Layout: odd numbers only, one bit each.  A window is WIN_WORDS 32-bit words
 // (2^19 odd numbers, a 2^20-wide range) held in shared memory.
+//   pass 0  sieve_starts: every base prime's first multiple in the range;
 //   pass 1  sieve_windows: each CTA clears a window, crosses off multiples
 //           of every odd base prime p (p^2 below the window end) with
 //           shared-memory atomics, writes the prime bitmap to global memory
-//           and its popcount;
-//   pass 2  scan_counts: exclusive scan of the window counts (one CTA);
-//   pass 3  compact: each CTA re-reads a window's bitmap and writes its
-//           primes at the window's offset, ordered by a block scan per round.
+//           and its popcount a chunk (CHUNK_WORDS);
+//   pass 2  scan_counts: exclusive scan of the chunk counts (one CTA);
+//   pass 3  compact: each CTA re-reads a chunk's bitmap and writes its
+//           primes at the chunk's offset, a warp a run of words.
+// Short ranges take quarter windows, so that every SM has some.
 // Base primes (all odd p <= sqrt(hi)) come from the same kernels: the odd
 // primes below 2^16 from a one-CTA sieve, the rest by sieving [3, sqrt(hi)].
 #include "ctd_internal.h"
@@ -28,8 +30,9 @@ namespace {
 
 constexpr uint32_t WIN_WORDS = 16384;                       // 64 KiB of shared memory
 constexpr uint64_t WIN_ODD = 32ull * WIN_WORDS;             // odd numbers per window
-constexpr int SIEVE_THREADS = 512;
-constexpr uint32_t SMALL_PRIMES = 256;                      // crossed off cooperatively by the CTA
+constexpr uint32_t CHUNK_WORDS = WIN_WORDS / SIEVE_WIN_CHUNKS;  // unit of the counts and the compaction; a short range's window
+constexpr int SIEVE_THREADS = 1024;
+constexpr int COMPACT_THREADS = 256;
 constexpr uint32_t LEVEL0_LIMIT = 65536;                    // level-0 base primes: odd p < 2^16
 
 #define CUDA_TRY(expr)                                                      \
@@ -42,21 +45,51 @@ constexpr uint32_t LEVEL0_LIMIT = 65536;                    // level-0 base prim
         }                                                                   \
     } while (0)
 
-// index (in odd steps from wlo) of the first odd multiple of p that is
-// >= max(p^2, wlo)
-__device__ __forceinline__ uint64_t first_index(uint32_t p, uint64_t wlo)
+// index (in odd steps from wlo) of the first odd multiple of p at or above wlo
+__device__ __forceinline__ uint64_t first_multiple(uint32_t p, uint64_t wlo)
 {
-    uint64_t pp = (uint64_t)p * p;
-    uint64_t m;
-    if (pp >= wlo) {
-        m = pp;
-    } else {
-        uint64_t r = wlo % p;
-        m = r ? wlo + (p - r) : wlo;
-        if (!(m & 1))
-            m += p;
-    }
+    const uint64_t r = wlo % p;
+    uint64_t m = r ? wlo + (p - r) : wlo;
+    if (!(m & 1))
+        m += p;
     return (m - wlo) >> 1;
+}
+
+// What a window needs of a base prime to find its first multiple there by
+// 32-bit arithmetic: the first multiple's index in the whole range, and
+// floor((2^32 - 1) / p).  A 64-bit division per prime and window -- and, for
+// the primes that a whole CTA crosses off, per thread -- was most of the
+// sieve's instructions.
+struct SieveStart {
+    uint32_t first, recip;
+};
+__global__ void __launch_bounds__(256) sieve_starts(uint64_t lo_odd, uint64_t last, const uint32_t *__restrict__ base,
+                                                    uint32_t nbase, SieveStart *__restrict__ starts)
+{
+    for (uint32_t k = blockIdx.x * 256 + threadIdx.x; k < nbase; k += gridDim.x * 256) {
+        const uint32_t p = base[k];
+        if ((uint64_t)p * p > last)
+            break;
+        starts[k] = SieveStart{(uint32_t)first_multiple(p, lo_odd), 0xffffffffu / p};
+    }
+}
+
+// index in the window at wlo = lo_odd + 2 off of the first multiple of p to
+// cross off: the first at or above max(p^2, wlo)
+template <bool STARTS>
+__device__ __forceinline__ uint64_t first_index(uint32_t p, uint64_t wlo, uint32_t off,
+                                                const SieveStart *__restrict__ starts, uint32_t k)
+{
+    const uint64_t pp = (uint64_t)p * p;
+    if (pp >= wlo)
+        return (pp - wlo) >> 1;
+    if (!STARTS)
+        return first_multiple(p, wlo);
+    const SieveStart s = starts[k];
+    // off mod p: the quotient is one short at most (2p fits 32 bits, or p > off)
+    uint32_t r = off - __umulhi(off, s.recip) * p;
+    r = r >= p ? r - p : r;
+    return s.first >= r ? s.first - r : s.first + (p - r);
 }
 
 // The wheel: the odd primes 3..31, whose multiples take most of a
@@ -79,18 +112,24 @@ __host__ __device__ constexpr uint32_t wheel_pattern(uint32_t q)
     return m;
 }
 
+// One CTA a window of win_words words.  Bound by the crossings in shared
+// memory: a warp crosses off up to 32 multiples an atomic, their banks at
+// random.
+template <bool STARTS>
 __global__ void __launch_bounds__(SIEVE_THREADS) sieve_windows(uint64_t lo_odd, uint64_t nodd, uint32_t nwin,
-                                                               const uint32_t *__restrict__ base, uint32_t nbase,
-                                                               uint32_t *__restrict__ bits, uint32_t *__restrict__ wcount)
+                                                               uint32_t win_words, const uint32_t *__restrict__ base,
+                                                               uint32_t nbase, const SieveStart *__restrict__ starts,
+                                                               uint32_t *__restrict__ bits, uint32_t *__restrict__ ccount)
 {
     extern __shared__ uint32_t sm[];
-    __shared__ uint32_t warp_sums[SIEVE_THREADS / 32];
-    const uint32_t tid = threadIdx.x, bd = blockDim.x;
+    __shared__ uint32_t chunk_count[WIN_WORDS / CHUNK_WORDS];
+    const uint32_t tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = bd >> 5;
+    const uint32_t win_odd = 32 * win_words;
     for (uint32_t w = blockIdx.x; w < nwin; w += gridDim.x) {
-        const uint64_t off = (uint64_t)w * WIN_ODD;
+        const uint64_t off = (uint64_t)w * win_odd;
         const uint64_t wlo = lo_odd + 2 * off;
-        const uint64_t len = (nodd - off) < WIN_ODD ? (nodd - off) : WIN_ODD;
-        const uint64_t whi = wlo + 2 * len;
+        const uint32_t len = (uint32_t)((nodd - off) < win_odd ? (nodd - off) : win_odd);
+        const uint64_t last = wlo + 2 * (uint64_t)(len - 1);  // (not one past it: that may be 2^64)
         {
             // bit b of word i is the odd number wlo + 2 (32 i + b); it is a
             // multiple of q iff its odd index g = (value - 1) / 2 is
@@ -107,7 +146,7 @@ __global__ void __launch_bounds__(SIEVE_THREADS) sieve_windows(uint64_t lo_odd, 
                 ph[k] = h >= gm ? h - gm : h + q - gm;
                 step[k] = (32u * bd) % q;
             }
-            for (uint32_t i = tid; i < WIN_WORDS; i += bd) {
+            for (uint32_t i = tid; i < win_words; i += bd) {
                 uint32_t v = 0;
 #pragma unroll
                 for (int k = 0; k < WHEEL; ++k) {
@@ -118,65 +157,85 @@ __global__ void __launch_bounds__(SIEVE_THREADS) sieve_windows(uint64_t lo_odd, 
                 sm[i] = v;
             }
         }
+        if (tid < WIN_WORDS / CHUNK_WORDS)
+            chunk_count[tid] = 0;
         __syncthreads();
         if (tid == 0 && wlo <= wheel_q(WHEEL - 1)) {
             // the wheel primes themselves are not composite
             for (int k = 0; k < WHEEL; ++k) {
                 const uint64_t q = wheel_q(k);
-                if (q >= wlo && q < whi) {
+                if (q >= wlo && q <= last) {
                     const uint64_t j = (q - wlo) >> 1;
                     sm[j >> 5] &= ~(1u << (j & 31));
                 }
             }
         }
         __syncthreads();
-        // small primes past the wheel: the whole CTA strides over each
-        // prime's multiples (base[] starts with the wheel primes 3..31)
-        const uint32_t nsmall = nbase < SMALL_PRIMES ? nbase : SMALL_PRIMES;
-        for (uint32_t k = WHEEL; k < nsmall; ++k) {
+        // primes past the wheel with 32 multiples and more in the window: a
+        // warp a prime (base[] starts with the wheel primes 3..31)
+        uint32_t k = WHEEL + warp;
+        for (; k < nbase; k += nwarps) {
             const uint32_t p = base[k];
-            if ((uint64_t)p * p >= whi)
+            if (p > win_odd / 32 || (uint64_t)p * p > last)
                 break;
-            const uint64_t j0 = first_index(p, wlo);
-            for (uint64_t j = j0 + (uint64_t)tid * p; j < len; j += (uint64_t)bd * p)
+            const uint64_t j0 = first_index<STARTS>(p, wlo, (uint32_t)off, starts, k);
+            if (j0 >= len)
+                continue;
+            for (uint32_t j = (uint32_t)j0 + lane * p; j < len; j += 32 * p)
                 atomicOr(&sm[j >> 5], 1u << (j & 31));
         }
-        // larger primes: one prime per thread
-        for (uint32_t k = nsmall + tid; k < nbase; k += bd) {
-            const uint32_t p = base[k];
-            if ((uint64_t)p * p >= whi)
-                break;
-            for (uint64_t j = first_index(p, wlo); j < len; j += p)
-                atomicOr(&sm[j >> 5], 1u << (j & 31));
+        // the others: a prime a thread.  The warps left the list at different
+        // places; the first prime above the bound is where this part starts
+        {
+            uint32_t a = WHEEL, b = nbase;
+            while (a < b) {
+                const uint32_t mid = (a + b) >> 1;
+                if (base[mid] <= win_odd / 32)
+                    a = mid + 1;
+                else
+                    b = mid;
+            }
+            k = a + tid;
+        }
+        // (the next prime is loaded while this one's multiples are crossed off)
+        uint32_t p = k < nbase ? base[k] : 0;
+        while (k < nbase && (uint64_t)p * p <= last) {
+            const uint32_t next = k + bd, pn = next < nbase ? base[next] : 0;
+            const uint64_t j0 = first_index<STARTS>(p, wlo, (uint32_t)off, starts, k);
+            if (j0 < len) {
+                uint32_t j = (uint32_t)j0;
+                do {
+                    atomicOr(&sm[j >> 5], 1u << (j & 31));
+                    j = p < len - j ? j + p : len;
+                } while (j < len);
+            }
+            k = next;
+            p = pn;
         }
         __syncthreads();
-        uint32_t cnt = 0;
-        uint32_t *out = bits + (uint64_t)w * WIN_WORDS;
-        for (uint32_t i = tid; i < WIN_WORDS; i += bd) {
-            uint32_t v = ~sm[i];
-            const uint64_t j = (uint64_t)i * 32;
-            if (j + 32 > len)
-                v = (j >= len) ? 0u : (v & ((1u << (uint32_t)(len - j)) - 1u));
-            out[i] = v;
-            cnt += __popc(v);
+        uint32_t *out = bits + (uint64_t)w * win_words;
+        for (uint32_t c = 0; c < win_words; c += CHUNK_WORDS) {
+            uint32_t cnt = 0;
+            for (uint32_t i = c + tid; i < c + CHUNK_WORDS; i += bd) {
+                uint32_t v = ~sm[i];
+                const uint32_t j = i * 32;
+                if (j + 32 > len)
+                    v = (j >= len) ? 0u : (v & ((1u << (len - j)) - 1u));
+                out[i] = v;
+                cnt += __popc(v);
+            }
+            cnt = __reduce_add_sync(0xffffffffu, cnt);
+            if (lane == 0)
+                atomicAdd(&chunk_count[c / CHUNK_WORDS], cnt);
         }
-        // block reduction of the window's prime count
-        for (int o = 16; o; o >>= 1)
-            cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        if ((tid & 31) == 0)
-            warp_sums[tid >> 5] = cnt;
         __syncthreads();
-        if (tid == 0) {
-            uint32_t s = 0;
-            for (uint32_t i = 0; i < bd / 32; ++i)
-                s += warp_sums[i];
-            wcount[w] = s;
-        }
+        if (tid < win_words / CHUNK_WORDS)
+            ccount[(uint64_t)w * (win_words / CHUNK_WORDS) + tid] = chunk_count[tid];
         __syncthreads();
     }
 }
 
-// exclusive scan of window counts into 64-bit offsets; offsets[nwin] = total
+// exclusive scan of chunk counts into 64-bit offsets; offsets[n] = total
 __global__ void __launch_bounds__(1024) scan_counts(const uint32_t *__restrict__ wcount, uint32_t nwin,
                                                     uint64_t *__restrict__ offsets)
 {
@@ -220,49 +279,54 @@ __global__ void __launch_bounds__(1024) scan_counts(const uint32_t *__restrict__
         offsets[nwin] = carry;
 }
 
+// A CTA a chunk of the bitmap, each warp a run of its words, 32 words at a
+// time: the words' primes are written in one stretch of a few hundred bytes,
+// a prime a lane and store.  With one CTA a window and a block scan for each
+// of its 32 rounds, the primes of a 2^26-wide range took 54 us to write.
 template <class T>
-__global__ void __launch_bounds__(SIEVE_THREADS) compact_windows(uint64_t lo_odd, uint32_t nwin,
-                                                                 const uint32_t *__restrict__ bits,
-                                                                 const uint64_t *__restrict__ offsets,
-                                                                 T *__restrict__ out, uint64_t capacity,
-                                                                 uint64_t out_base)
+__global__ void __launch_bounds__(COMPACT_THREADS) compact_chunks(uint64_t lo_odd, uint32_t nchunks,
+                                                                  const uint32_t *__restrict__ bits,
+                                                                  const uint64_t *__restrict__ offsets,
+                                                                  T *__restrict__ out, uint64_t capacity,
+                                                                  uint64_t out_base)
 {
-    __shared__ uint32_t warp_sums[SIEVE_THREADS / 32];
-    const uint32_t tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, warp = tid >> 5;
-    for (uint32_t w = blockIdx.x; w < nwin; w += gridDim.x) {
-        const uint64_t wlo = lo_odd + 2 * (uint64_t)w * WIN_ODD;
-        uint64_t run = out_base + offsets[w];
-        const uint32_t *wb = bits + (uint64_t)w * WIN_WORDS;
-        for (uint32_t r = 0; r < WIN_WORDS; r += bd) {
-            const uint32_t i = r + tid;
-            uint32_t v = i < WIN_WORDS ? wb[i] : 0u;
-            uint32_t c = __popc(v), x = c;
-            for (int o = 1; o < 32; o <<= 1) {
-                uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= (uint32_t)o)
-                    x += y;
-            }
-            if (lane == 31)
-                warp_sums[warp] = x;
-            __syncthreads();
-            uint32_t before = 0, total = 0;
-            for (uint32_t k = 0; k < bd / 32; ++k) {
-                uint32_t s = warp_sums[k];
-                if (k < warp)
-                    before += s;
-                total += s;
-            }
-            uint64_t pos = run + before + x - c;
-            while (v) {
-                const uint32_t b = __ffs(v) - 1;
-                v &= v - 1;
-                if (pos < capacity)
-                    out[pos] = (T)(wlo + 2 * ((uint64_t)i * 32 + b));
-                ++pos;
-            }
-            run += total;
-            __syncthreads();
+    constexpr int WARPS = COMPACT_THREADS / 32, ROUNDS = CHUNK_WORDS / COMPACT_THREADS;
+    __shared__ uint32_t warp_count[WARPS];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint32_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        const uint32_t first = warp * (32 * ROUNDS) + lane;  // word of round 0
+        const uint32_t *wb = bits + (uint64_t)c * CHUNK_WORDS + first;
+        uint32_t v[ROUNDS], cnt = 0;
+#pragma unroll
+        for (int r = 0; r < ROUNDS; ++r) {
+            v[r] = wb[32 * r];
+            cnt += __popc(v[r]);
         }
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (lane == 0)
+            warp_count[warp] = cnt;
+        __syncthreads();
+        uint64_t pos = out_base + offsets[c];
+        for (uint32_t k = 0; k < warp; ++k)
+            pos += warp_count[k];
+        const uint64_t value = lo_odd + 64 * ((uint64_t)c * CHUNK_WORDS + first);
+#pragma unroll
+        for (int r = 0; r < ROUNDS; ++r) {
+            const uint32_t n = __popc(v[r]);
+            uint32_t x = n;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                x += lane >= (uint32_t)o ? y : 0;
+            }
+            uint64_t at = pos + x - n;
+            for (uint32_t m = v[r]; m; m &= m - 1) {
+                if (at < capacity)
+                    out[at] = (T)(value + 64 * 32 * r + 2 * (__ffs(m) - 1));
+                ++at;
+            }
+            pos += __shfl_sync(0xffffffffu, x, 31);
+        }
+        __syncthreads();
     }
 }
 
@@ -278,8 +342,9 @@ __global__ void __launch_bounds__(1024) level0_primes(uint32_t *__restrict__ out
     __syncthreads();
     if (tid == 0)
         atomicOr(&sm[0], 1u);  // 1 is not prime
-    for (uint32_t k = 3 + 2 * tid; k < 256; k += 2 * blockDim.x)
-        for (uint32_t m = k * k; m < LEVEL0_LIMIT; m += 2 * k)
+    // (a warp a k: with a thread a k, the multiples of 3 alone took 176 us)
+    for (uint32_t k = 3 + 2 * (tid >> 5); k < 256; k += 2 * (blockDim.x >> 5))
+        for (uint32_t m = k * k + 2 * k * (tid & 31); m < LEVEL0_LIMIT; m += 64 * k)
             atomicOr(&sm[(m >> 1) >> 5], 1u << ((m >> 1) & 31));
     __syncthreads();
     // ordered compaction, one word per thread (NW = 1024 = blockDim)
@@ -329,10 +394,12 @@ struct SieveWorkspace {
     uint32_t nbase = 0;
     uint64_t base_limit = 0;
     size_t base_cap = 0;
+    SieveStart *d_starts = nullptr;  // one a base prime, of the last range sieved
+    size_t starts_cap = 0;
     // per-range scratch
     uint32_t *d_bits = nullptr;
     size_t bits_cap = 0;  // windows
-    uint32_t *d_wcount = nullptr;
+    uint32_t *d_wcount = nullptr;  // SIEVE_WIN_CHUNKS a window
     uint64_t *d_offsets = nullptr;
     size_t win_cap = 0;
     uint64_t *h_total = nullptr;  // pinned
@@ -355,6 +422,7 @@ void sieve_workspace_destroy(SieveWorkspace *ws)
     if (!ws)
         return;
     cudaFree(ws->d_base);
+    cudaFree(ws->d_starts);
     cudaFree(ws->d_bits);
     cudaFree(ws->d_wcount);
     cudaFree(ws->d_offsets);
@@ -373,8 +441,8 @@ static int ensure_windows(SieveWorkspace *ws, uint64_t nwin, std::string &err)
         ws->d_offsets = nullptr;
         ws->win_cap = 0;
         CUDA_TRY(cudaMalloc(&ws->d_bits, nwin * WIN_WORDS * sizeof(uint32_t)));
-        CUDA_TRY(cudaMalloc(&ws->d_wcount, nwin * sizeof(uint32_t)));
-        CUDA_TRY(cudaMalloc(&ws->d_offsets, (nwin + 1) * sizeof(uint64_t)));
+        CUDA_TRY(cudaMalloc(&ws->d_wcount, nwin * SIEVE_WIN_CHUNKS * sizeof(uint32_t)));
+        CUDA_TRY(cudaMalloc(&ws->d_offsets, (nwin * SIEVE_WIN_CHUNKS + 1) * sizeof(uint64_t)));
         ws->win_cap = nwin;
     }
     if (!ws->h_total)
@@ -382,10 +450,69 @@ static int ensure_windows(SieveWorkspace *ws, uint64_t nwin, std::string &err)
     return CTD_OK;
 }
 
-static int grid_for(const SieveWorkspace *ws, uint64_t nwin)
+static int ensure_starts(SieveWorkspace *ws, std::string &err)
 {
-    uint64_t g = (uint64_t)ws->sm_count * 3;  // three 64 KiB windows fit an SM
-    return (int)(nwin < g ? nwin : g);
+    if (ws->nbase > ws->starts_cap) {
+        cudaFree(ws->d_starts);
+        ws->d_starts = nullptr;
+        ws->starts_cap = 0;
+        CUDA_TRY(cudaMalloc(&ws->d_starts, ws->nbase * sizeof(SieveStart)));
+        ws->starts_cap = ws->nbase;
+    }
+    return CTD_OK;
+}
+
+// Launches the passes over the odd numbers lo_odd .. lo_odd + 2 (nodd - 1),
+// nodd > 0, into d_out[out_base ...]; the number of chunks is returned (the
+// count of primes is left at offsets[chunks]).  starts: room for one a base
+// prime, or null (the windows then divide for themselves).
+template <class T>
+static int launch_sieve(uint64_t lo_odd, uint64_t nodd, const uint32_t *d_base, uint32_t nbase, SieveStart *starts,
+                        uint32_t *bits, uint32_t *ccount, uint64_t *offsets, int sm_count, T *d_out, uint64_t capacity,
+                        uint64_t out_base, uint32_t *chunks, cudaStream_t st, std::string &err)
+{
+    // Whole windows where they give half the SMs one, else chunks as windows;
+    // 1024 threads a window while the windows are few.  A 2^27-wide range at
+    // 2^40 (82,000 base primes a window): 140 us with its 128 whole windows,
+    // 226 with 512 chunks; a 2^26-wide one at 2^33: 80 us with 256 chunks of
+    // 512 threads, 84 with 1024 and 105 with 64 whole windows; a 2^20-wide one
+    // 57 us with 1024 threads a chunk and 68 with 512; a 2^28-wide one 194 us
+    // with 1024 threads a whole window, a 2^29-wide one 355, and 335 with 512.
+    const uint64_t full = (nodd + WIN_ODD - 1) / WIN_ODD;
+    const uint32_t win_words = 2 * full >= (uint64_t)sm_count ? WIN_WORDS : CHUNK_WORDS;
+    const uint64_t nwin = (nodd + 32ull * win_words - 1) / (32ull * win_words);
+    const uint32_t nchunks = (uint32_t)(nwin * (win_words / CHUNK_WORDS));
+    const int threads = nwin <= (uint64_t)sm_count * (win_words == WIN_WORDS ? 2 : 1) ? SIEVE_THREADS : SIEVE_THREADS / 2;
+    const size_t smem = win_words * sizeof(uint32_t);
+    if (nodd >> 32)
+        starts = nullptr;  // offsets in the range are 32-bit
+    // a function attribute belongs to the current device: set it on every
+    // call (a host-side call, no stream work), so a context on any device
+    // launches with it
+    CUDA_TRY(cudaFuncSetAttribute(starts ? sieve_windows<true> : sieve_windows<false>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(WIN_WORDS * sizeof(uint32_t))));
+    if (starts) {
+        const uint32_t blocks = (nbase + 255) / 256;
+        sieve_starts<<<blocks < (uint32_t)sm_count * 4 ? blocks : (uint32_t)sm_count * 4, 256, 0, st>>>(
+            lo_odd, lo_odd + 2 * (nodd - 1), d_base, nbase, starts);
+        CUDA_TRY(cudaGetLastError());
+        note_kernel_launch();
+        sieve_windows<true><<<(unsigned)nwin, threads, smem, st>>>(lo_odd, nodd, (uint32_t)nwin, win_words, d_base, nbase,
+                                                                   starts, bits, ccount);
+    } else {
+        sieve_windows<false><<<(unsigned)nwin, threads, smem, st>>>(lo_odd, nodd, (uint32_t)nwin, win_words, d_base,
+                                                                    nbase, starts, bits, ccount);
+    }
+    CUDA_TRY(cudaGetLastError());
+    note_kernel_launch();
+    scan_counts<<<1, 1024, 0, st>>>(ccount, nchunks, offsets);
+    CUDA_TRY(cudaGetLastError());
+    note_kernel_launch();
+    compact_chunks<T><<<nchunks, COMPACT_THREADS, 0, st>>>(lo_odd, nchunks, bits, offsets, d_out, capacity, out_base);
+    CUDA_TRY(cudaGetLastError());
+    note_kernel_launch();
+    *chunks = nchunks;
+    return CTD_OK;
 }
 
 // odd primes in [lo_odd, lo_odd + 2*nodd) into out[out_base ...], counts in ws
@@ -398,31 +525,22 @@ static int sieve_odd(SieveWorkspace *ws, uint64_t lo_odd, uint64_t nodd, const u
     if (!nodd)
         return CTD_OK;
     const uint64_t nwin = (nodd + WIN_ODD - 1) / WIN_ODD;
-    if (nwin > 0xffffffffull) {
+    if (nwin * SIEVE_WIN_CHUNKS > 0x7fffffffull) {
         err = "sieve range too large";
         return CTD_ERR_INVALID_ARGUMENT;
     }
     int rc = ensure_windows(ws, nwin, err);
     if (rc)
         return rc;
-    const size_t smem = WIN_WORDS * sizeof(uint32_t);
-    // a function attribute belongs to the current device: set it on every
-    // call (a host-side call, no stream work), so a context on any device
-    // launches with it
-    CUDA_TRY(cudaFuncSetAttribute(sieve_windows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int grid = grid_for(ws, nwin);
-    sieve_windows<<<grid, SIEVE_THREADS, smem, st>>>(lo_odd, nodd, (uint32_t)nwin, d_base, nbase, ws->d_bits,
-                                                    ws->d_wcount);
-    CUDA_TRY(cudaGetLastError());
-    note_kernel_launch();
-    scan_counts<<<1, 1024, 0, st>>>(ws->d_wcount, (uint32_t)nwin, ws->d_offsets);
-    CUDA_TRY(cudaGetLastError());
-    note_kernel_launch();
-    compact_windows<T><<<grid, SIEVE_THREADS, 0, st>>>(lo_odd, (uint32_t)nwin, ws->d_bits, ws->d_offsets, d_out,
-                                                       capacity, out_base);
-    CUDA_TRY(cudaGetLastError());
-    note_kernel_launch();
-    CUDA_TRY(cudaMemcpyAsync(ws->h_total, ws->d_offsets + nwin, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    rc = ensure_starts(ws, err);
+    if (rc)
+        return rc;
+    uint32_t chunks = 0;
+    rc = launch_sieve<T>(lo_odd, nodd, d_base, nbase, ws->d_starts, ws->d_bits, ws->d_wcount, ws->d_offsets,
+                         ws->sm_count, d_out, capacity, out_base, &chunks, st, err);
+    if (rc)
+        return rc;
+    CUDA_TRY(cudaMemcpyAsync(ws->h_total, ws->d_offsets + chunks, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     *count = *ws->h_total;
     return CTD_OK;
@@ -525,18 +643,14 @@ int sieve_prepare_base(SieveWorkspace *ws, uint64_t hi, cudaStream_t st, std::st
 {
     if (hi < 3)
         return CTD_OK;
-    return ensure_base(ws, isqrt64(hi - 1), st, err);
+    const int rc = ensure_base(ws, isqrt64(hi - 1), st, err);
+    return rc ? rc : ensure_starts(ws, err);
 }
 
 int sieve_prepare_windows(SieveWorkspace *ws, uint64_t max_width, std::string &err)
 {
     const uint64_t nwin = (max_width / 2 + 1 + WIN_ODD - 1) / WIN_ODD + 1;
-    int rc = ensure_windows(ws, nwin, err);
-    if (rc)
-        return rc;
-    const size_t smem = WIN_WORDS * sizeof(uint32_t);
-    CUDA_TRY(cudaFuncSetAttribute(sieve_windows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return CTD_OK;
+    return ensure_windows(ws, nwin, err);
 }
 
 uint64_t sieve_state_key(const SieveWorkspace *ws)
@@ -544,7 +658,7 @@ uint64_t sieve_state_key(const SieveWorkspace *ws)
     // FNV-1a over what sieve_odd_async's launches take besides the range
     const uint64_t parts[] = {(uint64_t)(uintptr_t)ws->d_base, ws->nbase, (uint64_t)(uintptr_t)ws->d_bits,
                               (uint64_t)(uintptr_t)ws->d_wcount, (uint64_t)(uintptr_t)ws->d_offsets,
-                              (uint64_t)ws->sm_count};
+                              (uint64_t)(uintptr_t)ws->d_starts, (uint64_t)ws->sm_count};
     uint64_t h = 1469598103934665603ull;
     for (uint64_t x : parts)
         for (int b = 0; b < 8; ++b) {
@@ -560,29 +674,20 @@ int sieve_odd_async(SieveWorkspace *ws, uint64_t lo, uint64_t hi, uint64_t *d_ou
     const uint64_t lo_odd = lo < 3 ? 3 : (lo | 1);
     const uint64_t nodd = lo_odd < hi ? (hi - lo_odd + 1) / 2 : 0;
     const uint64_t nwin = nodd ? (nodd + WIN_ODD - 1) / WIN_ODD : 0;
-    if (nwin > ws->win_cap || !ws->d_base) {
+    if (nwin > ws->win_cap || !ws->d_base || ws->nbase > ws->starts_cap) {
         err = "sieve scratch not prepared for this segment";
         return CTD_ERR_INVALID_ARGUMENT;
     }
-    *count_out = ws->d_offsets + nwin;
     if (!nwin) {  // empty: a zero count
+        *count_out = ws->d_offsets;
         CUDA_TRY(cudaMemsetAsync(ws->d_offsets, 0, sizeof(uint64_t), st));
         return CTD_OK;
     }
-    const size_t smem = WIN_WORDS * sizeof(uint32_t);
-    const int grid = grid_for(ws, nwin);
-    sieve_windows<<<grid, SIEVE_THREADS, smem, st>>>(lo_odd, nodd, (uint32_t)nwin, ws->d_base, ws->nbase, ws->d_bits,
-                                                    ws->d_wcount);
-    CUDA_TRY(cudaGetLastError());
-    scan_counts<<<1, 1024, 0, st>>>(ws->d_wcount, (uint32_t)nwin, ws->d_offsets);
-    CUDA_TRY(cudaGetLastError());
-    compact_windows<uint64_t><<<grid, SIEVE_THREADS, 0, st>>>(lo_odd, (uint32_t)nwin, ws->d_bits, ws->d_offsets,
-                                                              d_out, capacity, 0);
-    CUDA_TRY(cudaGetLastError());
-    note_kernel_launch();
-    note_kernel_launch();
-    note_kernel_launch();
-    return CTD_OK;
+    uint32_t chunks = 0;
+    const int rc = launch_sieve<uint64_t>(lo_odd, nodd, ws->d_base, ws->nbase, ws->d_starts, ws->d_bits, ws->d_wcount,
+                                          ws->d_offsets, ws->sm_count, d_out, capacity, 0, &chunks, st, err);
+    *count_out = ws->d_offsets + chunks;
+    return rc;
 }
 
 // ----------------------------------------------- fixed-scratch variant
@@ -610,8 +715,6 @@ int sieve_range_scratch(const SieveScratch &sc, int sm_count, uint64_t lo, uint6
     *count = 0;
     if (hi <= lo)
         return CTD_OK;
-    const size_t smem = WIN_WORDS * sizeof(uint32_t);
-    CUDA_TRY(cudaFuncSetAttribute(sieve_windows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     uint64_t out_base = 0;
     if (lo <= 2 && hi > 2) {
         if (capacity > 0) {  // the u64 value 2, little-endian
@@ -636,36 +739,21 @@ int sieve_range_scratch(const SieveScratch &sc, int sm_count, uint64_t lo, uint6
     if (bwin) {
         const uint64_t b_lo = LEVEL0_LIMIT + 1;
         const uint64_t b_nodd = (limit - b_lo) / 2 + 1;
-        const int grid = (int)std::min<uint64_t>(bwin, (uint64_t)sm_count * 3);
-        sieve_windows<<<grid, SIEVE_THREADS, smem, st>>>(b_lo, b_nodd, (uint32_t)bwin, sc.base, nlevel0, sc.bits,
-                                                         sc.wcount);
-        CUDA_TRY(cudaGetLastError());
-        scan_counts<<<1, 1024, 0, st>>>(sc.wcount, (uint32_t)bwin, sc.offsets);
-        CUDA_TRY(cudaGetLastError());
-        compact_windows<uint32_t><<<grid, SIEVE_THREADS, 0, st>>>(b_lo, (uint32_t)bwin, sc.bits, sc.offsets, sc.base,
-                                                                  sc.base_cap - 1, nlevel0);
-        CUDA_TRY(cudaGetLastError());
-        note_kernel_launch();
-        note_kernel_launch();
-        note_kernel_launch();
+        uint32_t chunks = 0;
+        const int rc = launch_sieve<uint32_t>(b_lo, b_nodd, sc.base, nlevel0, nullptr, sc.bits, sc.wcount, sc.offsets,
+                                              sm_count, sc.base, sc.base_cap - 1, nlevel0, &chunks, st, err);
+        if (rc)
+            return rc;
     }
     // the range itself, against every base prime (the sentinel tail stops the scan)
     const uint64_t nodd = (hi - lo_odd + 1) / 2;
-    const uint64_t nwin = (nodd + WIN_ODD - 1) / WIN_ODD;
-    const int grid = (int)std::min<uint64_t>(nwin, (uint64_t)sm_count * 3);
-    sieve_windows<<<grid, SIEVE_THREADS, smem, st>>>(lo_odd, nodd, (uint32_t)nwin, sc.base, sc.base_cap, sc.bits,
-                                                     sc.wcount);
-    CUDA_TRY(cudaGetLastError());
-    scan_counts<<<1, 1024, 0, st>>>(sc.wcount, (uint32_t)nwin, sc.offsets);
-    CUDA_TRY(cudaGetLastError());
-    compact_windows<uint64_t><<<grid, SIEVE_THREADS, 0, st>>>(lo_odd, (uint32_t)nwin, sc.bits, sc.offsets, d_out,
-                                                              capacity, out_base);
-    CUDA_TRY(cudaGetLastError());
-    note_kernel_launch();
-    note_kernel_launch();
-    note_kernel_launch();
+    uint32_t chunks = 0;
+    const int rc = launch_sieve<uint64_t>(lo_odd, nodd, sc.base, (uint32_t)sc.base_cap, nullptr, sc.bits, sc.wcount,
+                                          sc.offsets, sm_count, d_out, capacity, out_base, &chunks, st, err);
+    if (rc)
+        return rc;
     uint64_t total = 0;
-    CUDA_TRY(cudaMemcpyAsync(&total, sc.offsets + nwin, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaMemcpyAsync(&total, sc.offsets + chunks, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     *count = out_base + total;
     return CTD_OK;

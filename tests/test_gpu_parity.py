@@ -278,3 +278,18 @@ def test_the_prime_2_alone(eng, family, param, n0, terms):
     # one thread a term; [0, 3) holds no odd prime
     got = run_gpu(eng, family, param, n0, n0 + terms, 0, 3, 2)
     assert text(got) == O.trial_factor(family, param, n0, n0 + terms, 0, 3, 2, threads=1).format()
+
+
+@pytest.mark.parametrize("lo", [0, (1 << 18) - 30, (1 << 36) + 1, (1 << 50) + 12345, (1 << 62) - 99])
+@pytest.mark.parametrize("width", [1, 62, (1 << 18) - 2, 1 << 18, (1 << 18) + 2, (1 << 20) + (1 << 18) + 64])
+def test_sieve_chunk_edges(eng, lo, width):
+    assert np.array_equal(eng.sieve(lo, lo + width), O.sieve(lo, lo + width))
+
+
+@pytest.mark.parametrize("lo", [0, (1 << 33) + 5])
+def test_sieve_whole_and_quarter_windows(eng, lo):
+    # two whole windows an SM and more, against parts that go by quarter windows
+    sms = eng.device_info()["sm_count"]
+    hi = lo + 2 * sms * (1 << 20) + 777
+    mid = (lo + hi) // 2
+    assert np.array_equal(eng.sieve(lo, hi), np.concatenate([eng.sieve(lo, mid), eng.sieve(mid, hi)]))
