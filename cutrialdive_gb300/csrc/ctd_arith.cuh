@@ -111,12 +111,16 @@ struct MontT {
     CTD_HD static uint64_t neg_inverse(uint64_t p)
     {
         // Newton-Hensel lifting: x <- x(2 - px) doubles the correct low bits;
-        // x = p is correct to 3 bits for odd p (p*p = 1 mod 8).
-        uint64_t x = p;
+        // x = p is correct to 3 bits for odd p (p*p = 1 mod 8).  Four steps
+        // on 32-bit words (48 bits, so all 32), the last on 64.
+        const uint32_t p32 = (uint32_t)p;
+        uint32_t x = p32;
         #pragma unroll
-        for (int i = 0; i < 5; ++i)
-            x *= 2 - p * x;
-        return (uint64_t)0 - x;
+        for (int i = 0; i < 4; ++i)
+            x *= 2u - p32 * x;
+        uint64_t y = x;
+        y *= 2 - p * y;
+        return (uint64_t)0 - y;
     }
 
     // Everything but r2: enough for pow2/pow/mul/from and for mul(X, y)
@@ -245,6 +249,34 @@ struct MontT {
         return r;
     }
 };
+// 2^-x mod p for odd p (NARROW: p < 2^40), pinv = -p^-1 mod 2^64.  2^-f is (1 + m p) / 2^f
+// with m = pinv mod 2^f, for f below 64 at once; with X(e) = 2^(64-e) mod p the
+// Montgomery product of X(a) and X(b) is X(a+b), halving X(e) gives X(e+1), and
+// X(64+f) = 2^-f: the seven leading bits of a longer x cost that one product,
+// each further bit a squaring, and nothing needs R mod p, a 64-bit division.
+// (2^(p-1-x) by Fermat takes a squaring for every bit of p.)
+template <bool NARROW>
+CTD_HD uint64_t half_power(uint64_t p, uint64_t pinv, uint64_t x)
+{
+    MontT<NARROW> m;
+    m.p = p;
+    m.pinv = pinv;
+    const int bits = 64 - clz64(x | 64);       // 7 and more
+    const int rest = x < 64 ? 0 : bits - 7;    // bits of x after the leading ones
+    const uint32_t f = (uint32_t)(x >> rest) & 63;
+    const uint64_t mask = (1ull << f) - 1, mm = pinv & mask;
+    const uint64_t lo = mm * p + 1, hi = mulhi64(mm, p) + (lo == 0);
+    uint64_t r = f ? (hi << (64 - f)) | (lo >> f) : lo;
+    if (x < 64)
+        return r;
+    for (int b = rest - 1; b >= 0; --b) {
+        r = m.mul(r, r);
+        if ((x >> b) & 1)
+            r = (r >> 1) + ((r & 1) ? (p >> 1) + 1 : 0);
+    }
+    return m.mul(r, 1);
+}
+
 using Mont = MontT<false>;
 using MontN = MontT<true>;  // p < 2^40
 constexpr uint64_t MONT_NARROW_LIMIT = 1ull << 40;

@@ -526,12 +526,12 @@ __device__ __forceinline__ uint64_t redc32(uint64_t u, uint32_t plo, uint32_t ph
 template <uint32_t FAM>
 __device__ __forceinline__ void run_doubling(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
 {
-    Mont m;
-    m.init_lite(p);
     const uint64_t target = (FAM == PROTH) ? p - 1 : 1;
     const uint64_t steps = e - s - 1;
     // u(s) = k 2^s mod p, for the per-step walks
     auto start = [&]() {
+        Mont m;
+        m.init_lite(p);
         const uint64_t U = m.pow2(s);  // 2^s in Montgomery form
         if (FAM == MERSENNE)
             return m.from(U);
@@ -546,8 +546,9 @@ __device__ __forceinline__ void run_doubling(const JobView &job, uint64_t p, uin
         // Term n + j of a block starting at n is a zero iff w(n) = target 2^j.
         const uint64_t k = FAM == MERSENNE ? 1 : (job.param < p ? job.param : job.param % p);
         const uint64_t wt = (FAM == PROTH) ? (k ? p - k : 0) : k;  // target of w
+        const uint64_t pinv = Mont::neg_inverse(p);
         const uint64_t sr = s < p - 1 ? s : s % (p - 1);
-        uint64_t w = m.from(m.pow2(p - 1 - sr));  // 2^-s mod p (Fermat)
+        uint64_t w = p < MONT_NARROW_LIMIT ? half_power<true>(p, pinv, sr) : half_power<false>(p, pinv, sr);  // 2^-s
         const uint64_t nb = (e - s) / BS;
         uint32_t tlo[BS];
         uint64_t t = wt;
@@ -556,7 +557,7 @@ __device__ __forceinline__ void run_doubling(const JobView &job, uint64_t p, uin
             tlo[j] = (uint32_t)t;
             t = add63(t, t, p);
         }
-        const uint32_t plo = (uint32_t)p, phi = (uint32_t)(p >> 32), pinv32 = (uint32_t)m.pinv;
+        const uint32_t plo = (uint32_t)p, phi = (uint32_t)(p >> 32), pinv32 = (uint32_t)pinv;
         const uint32_t one = (uint32_t)(p & 1);
         const uint64_t at0 = s - job.n0;  // index of the first term
         auto giant = [&](uint64_t x) { return redc32(x, plo, phi, pinv32, one); };
@@ -752,15 +753,18 @@ __device__ __forceinline__ uint32_t aggregated_increment(uint32_t *counter, uint
 // p-1 for Proth, v == 1 for Riesel).  The congruence is linear in k: p
 // divides S(k) iff k = -+2^-n (mod p), so the zeros in [s, e) are k0, k0 + p,
 // k0 + 2p, ... from the first k0 >= s of that class -- one power of 2 per
-// prime and no walk; the pushed (k, p) pairs are exactly the walk's.
+// prime and no walk; the pushed (k, p) pairs are exactly the walk's.  The
+// primes of a 2^26-wide segment at 2^32, n = 12345: 243 us with 2^(p-1-n) (a
+// squaring a bit of p and R mod p), 73 us with half_power (610 instructions a prime,
+// most of them eight narrow products).
 // CTD_VARIANT_WALK keeps the term-by-term walk (a second algorithm for the
 // cross-checks).
 template <uint32_t FAM>
 __device__ __forceinline__ void run_fixed_n(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
 {
-    Mont m;
-    m.init_lite(p);
     if (job.variant == CTD_VARIANT_WALK) {
+        Mont m;
+        m.init_lite(p);
         const uint64_t C = m.pow2(job.param);  // 2^n in Montgomery form
         const uint64_t c = m.from(C);
         const uint64_t v = m.mul(C, s < p ? s : s % p);  // plain s*2^n mod p
@@ -771,9 +775,10 @@ __device__ __forceinline__ void run_fixed_n(const JobView &job, uint64_t p, uint
             walk_target(v, target, p, s - job.n0, e - s - 1, job.fb, [p, c](uint64_t x) { return addmod(x, c, p); });
         return;
     }
-    // u = 2^-n = 2^(p-1-(n mod (p-1))) (Fermat; p odd, so 2 is invertible)
+    // u = 2^-n, n mod p - 1 (Fermat; p odd, so 2 is invertible)
     const uint64_t nr = job.param < p - 1 ? job.param : job.param % (p - 1);
-    const uint64_t u = m.from(m.pow2(p - 1 - nr));
+    const uint64_t pinv = Mont::neg_inverse(p);
+    const uint64_t u = p < MONT_NARROW_LIMIT ? half_power<true>(p, pinv, nr) : half_power<false>(p, pinv, nr);
     const uint64_t k0 = FAM == PROTH_FIXED_N ? p - u : u;  // u in [1, p-1]
     const uint64_t sr = s < p ? s : s % p;
     const uint64_t off = k0 >= sr ? k0 - sr : p - sr + k0;  // first k >= s with k = k0 (mod p)
