@@ -342,11 +342,10 @@ class Engine:
                   segment_length: int = 0, callback=None) -> None:
         """ctd_run_plain with a host factors buffer (updated in place)."""
         def _cb(_user, prog, snapshot):
-            if callback is None:
-                return N.CTD_CB_CONTINUE
             return int(callback(prog.contents, bool(snapshot)) or 0)
 
-        cb = N.PROGRESS_CB(_cb)
+        # a null callback lets the segments follow one another without a wait
+        cb = N.PROGRESS_CB(_cb) if callback is not None else N.PROGRESS_CB()
         rc = self._L.ctd_run_plain(self._h, ctypes.byref(job), buf.counts.ctypes.data_as(N.p32),
                                    buf.factors.ctypes.data_as(N.p64), resume_after_prime, segment_length, cb, None)
         self._check(rc, "ctd_run_plain")

@@ -222,6 +222,7 @@ int tuning_slot(uint32_t family) { return family < 9 ? (int)family : 9; }
 constexpr uint32_t DEFAULT_ITEMS_PER_THREAD = 8;
 constexpr uint32_t DEFAULT_MIN_TILE = 4096;
 constexpr uint32_t DEFAULT_SEGMENT_LOG2 = 26;
+constexpr uint32_t LONG_SEGMENT_LOG2 = 28;
 
 int bit_length(uint64_t x) { return x ? 64 - __builtin_clzll(x) : 0; }
 
@@ -313,10 +314,30 @@ uint32_t refine_q_of(const ctd_ctx *ctx, uint32_t family, int bits)
     return t ? t->refine_q : 0;
 }
 
-uint64_t default_segment(const ctd_ctx *ctx, uint32_t family, int bits)
+// The segment length of a call that names none.  Where no callback sees the
+// segments they are 2^28 wide: a segment costs a wait for its prime count, up
+// to 17 launches and their last waves (Proth, 100,000 terms, a 2^30-wide
+// range: 32.7 ms in segments of 2^26, 29.9 of 2^28, 29.2 of 2^30; fixed n 2.73,
+// 1.98, 1.73), if the device has room for twice what the context has to
+// allocate for them (the primes and the class buffers, 69 bytes a prime).
+uint64_t default_segment(const ctd_ctx *ctx, uint32_t family, int bits, uint64_t f0, uint64_t f1, bool seen)
 {
     const ctd_tuning *t = tuning_of(ctx, family, bits);
-    return 1ull << (t && t->segment_log2 ? t->segment_log2 : DEFAULT_SEGMENT_LOG2);
+    if (t && t->segment_log2)
+        return 1ull << t->segment_log2;
+    const uint64_t shorter = 1ull << DEFAULT_SEGMENT_LOG2, longer = 1ull << LONG_SEGMENT_LOG2;
+    if (seen || f1 <= f0 || f1 - f0 <= shorter)
+        return shorter;
+    const uint64_t primes = prime_count_upper_bound(f0, f1 - f0 > longer ? f0 + longer : f1);
+    const bool classes = family == CTD_PROTH || family == CTD_RIESEL || family == CTD_MERSENNE;
+    if (primes > ctx->primes_cap || (classes && primes > ctx->rs->cap)) {
+        size_t free_bytes = 0, total = 0;
+        if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || free_bytes / (2 * 69) < primes) {
+            (void)cudaGetLastError();
+            return shorter;
+        }
+    }
+    return longer;
 }
 
 JobView make_view(const ctd_job *job, uint32_t *d_counts, uint64_t *d_factors)
@@ -850,7 +871,8 @@ int ctd_run_plain(ctd_ctx *ctx, const ctd_job *job, uint32_t *counts_inout, uint
     }
     // tuning by prime width: the job's first prime sets the segment length,
     // each segment's first prime its launch shape and step forms
-    const uint64_t seg = segment_length ? segment_length : default_segment(ctx, job->family, bit_length(f0));
+    const uint64_t seg = segment_length ? segment_length
+                                         : default_segment(ctx, job->family, bit_length(f0), f0, f1, cb != nullptr);
     uint64_t last_prime = resume_after_prime;
     uint64_t primes_done = 0;
     for (uint64_t fx = f0, fy = (f1 - f0 > seg) ? f0 + seg : f1; fx < f1;
@@ -876,15 +898,15 @@ int ctd_run_plain(ctd_ctx *ctx, const ctd_job *job, uint32_t *counts_inout, uint
             rc = launch_residues(view, ctx->d_primes, np, grid, block, st, err, ctx->rs);
             if (rc)
                 return fail(ctx, rc, err);
-            uint64_t lp = 0;
-            CTX_CUDA(cudaMemcpyAsync(&lp, ctx->d_primes + np - 1, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-            CTX_CUDA(cudaStreamSynchronize(st));
-            last_prime = lp;
             primes_done += np;
-        } else {
-            CTX_CUDA(cudaStreamSynchronize(st));
         }
         if (cb) {
+            // (without a callback nothing waits here: the next segment's
+            // sieve is queued behind this one's walk)
+            if (np)
+                CTX_CUDA(cudaMemcpyAsync(&last_prime, ctx->d_primes + np - 1, sizeof(uint64_t), cudaMemcpyDeviceToHost,
+                                         st));
+            CTX_CUDA(cudaStreamSynchronize(st));
             ctd_progress prog;
             prog.segment_end = fy;
             prog.last_prime = last_prime;

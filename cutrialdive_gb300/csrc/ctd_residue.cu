@@ -755,8 +755,8 @@ __device__ __forceinline__ uint32_t aggregated_increment(uint32_t *counter, uint
 // k0 + 2p, ... from the first k0 >= s of that class -- one power of 2 per
 // prime and no walk; the pushed (k, p) pairs are exactly the walk's.  The
 // primes of a 2^26-wide segment at 2^32, n = 12345: 243 us with 2^(p-1-n) (a
-// squaring a bit of p and R mod p), 73 us with half_power (610 instructions a prime,
-// most of them eight narrow products).
+// squaring a bit of p and R mod p), 73 us with half_power (610 instructions a
+// prime, most of them eight narrow products).
 // CTD_VARIANT_WALK keeps the term-by-term walk (a second algorithm for the
 // cross-checks).
 template <uint32_t FAM>

@@ -177,7 +177,8 @@ int ctd_check_job(const ctd_job *job);
  * result; the reference's device push keeps whichever arrive first and both
  * report the excess (src/factors_buffer.hpp:62-75).  Primes p <= resume_after_prime are
  * skipped (src/trial_factoring.cuh:404).  segment_length 0 = the tuned
- * length for the job's family and first prime width (2^26 untuned).  Across
+ * length for the job's family and first prime width (untuned 2^26; 2^28
+ * without a callback, where the device has the room).  Across
  * the host link the call moves only what it must: an all-zero resume state
  * is cleared on the device instead of uploaded, and the counts come back
  * with the occupied slots only (the host slots past a count stay zero).
