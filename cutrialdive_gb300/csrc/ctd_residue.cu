@@ -1654,11 +1654,11 @@ __device__ __noinline__ uint32_t smarandache_blocks32(const JobView &job, Mont32
     return smarandache_exact32(job.fb, job.n0, p, x, M, Ms, m, steps);
 }
 
-// ---- blocks of J terms, 2^30 <= p < 2^52
+// ---- blocks of J terms, 2^30 <= p < 2^44
 // Within a digit class Y(m) = (M-1)^2 S(m) + t(m), t(m) = (M-1) m + M, obeys
 // Y(m+1) = M Y(m): p divides S(m) iff Y = t(m) (mod p) (p > M, so M - 1 is a
 // unit).  A block holds Y < 4p for its first term; term m + i is a zero only
-// if Y M^i - t(m+i) = k p with -t / p <= k < 4 M^i, and (Y M^i - t) p^-1 mod
+// if Y M^i - t(m+i) = k p with k < 4 M^i and -k not above t / p, and (Y M^i - t) p^-1 mod
 // 2^32 = k: one multiply-add of Y's low word and one compare a term, and only
 // every J-th Y is computed, W = M^J as an integer, Y W - q p in 64 bits:
 //   J = 2, 3: W <= 2^29 and q = mulhi(Y >> (sh-29), floor(W 2^(sh+3) / p)),
@@ -1671,33 +1671,37 @@ __device__ __noinline__ uint32_t smarandache_blocks32(const JobView &job, Mont32
 // A walk of S itself adds m in the wide product and compares with 0, p, 2p.
 // Bound by the multiply pipe (a wide product with a 64-bit sum takes nearly
 // three slots).  The primes of a 2^25-wide range at 2^34: base 10, n = 2001 ..
-// 8999 (J = 2), 4.43 ms, 6.9 with the walk of S; base 7, n = 20001 .. 24321
-// (J = 1), 4.32 and 4.50.
-__device__ __noinline__ uint64_t smarandache_exact64(FactorsView fb, uint64_t n0, uint64_t p, uint64_t Y, uint32_t M, uint64_t Ms,
-                                                     uint64_t m, uint32_t count)
+// 8999 (J = 2), 4.40 ms, 6.8 with the walk of S; base 7, n = 20001 .. 24321
+// (J = 1), 3.99 and 4.50.
+__device__ __noinline__ uint64_t smarandache_exact64(FactorsView fb, uint64_t n0, uint64_t p, uint64_t Y, uint64_t t,
+                                                     uint64_t dt, uint32_t M, uint64_t Ms, uint64_t m, uint32_t count)
 {
     while (Y >= p)
         Y -= p;
-    uint64_t t = ((uint64_t)(M - 1) * m + M) % p;
+    t %= p;
 #pragma unroll 1
     for (uint32_t i = 0; i < count; ++i) {
         if (Y == t)
             push(fb, m + i - n0, p);
-        t = addmod(t, M - 1, p);
+        t = addmod(t, dt, p);
         Y = Y * M - mulhi64(Y, Ms) * p;
         Y = Y >= p ? Y - p : Y;
     }
     return Y;
 }
 
-// The terms m .. m + steps - 1 of one digit class from Y = Y(m) < 2p; returns
-// Y(m + steps) below p.  Ms = floor(M 2^64 / p), Ws = floor(M^J 2^64 / p).
+// The terms m .. m + steps - 1 (steps < 2^20) of one digit class from
+// Y = Y(m) < 2p; returns Y(m + steps) below p.  Ms = floor(M 2^64 / p),
+// Ws = floor(M^J 2^64 / p).  Y and its targets may carry a common factor (the
+// denominator of S): the targets are t, t + dt, t + 2 dt, ... as integers,
+// t, dt < p, so -k is at most the number of terms.
 template <int J>
 __device__ __noinline__ uint64_t smarandache_blocks64(const JobView &job, uint64_t p, uint32_t pinv, uint64_t Y,
-                                                         uint32_t M, uint64_t Ms, uint64_t Ws, uint64_t m, uint64_t steps)
+                                                         uint64_t t, uint64_t dt, uint32_t M, uint64_t Ms, uint64_t Ws,
+                                                         uint64_t m, uint32_t steps)
 {
     constexpr int GROUP = J == 1 ? 8 : SM_GROUP;
-    const uint64_t groups = steps / (GROUP * J);
+    const uint32_t groups = steps / (GROUP * J);
     if (groups) {
         const int sh = 63 - clz64(p);
         const uint64_t np = (uint64_t)0 - p;
@@ -1705,18 +1709,17 @@ __device__ __noinline__ uint64_t smarandache_blocks64(const JobView &job, uint64
         const uint32_t W = J == 1 ? M : J == 2 ? M * M : M * M * M;
         const uint32_t R = (uint32_t)(Ws >> (61 - sh));
         const float Rf = __ull2float_rd(Ws) * __int_as_float((127 - 64 + sh - 22) << 23);
-        const uint32_t below = (uint32_t)(((uint64_t)(M - 1) * (m + steps) + M) / p) + 1;
-        const uint32_t dt = (M - 1) * pinv * J;
+        const uint32_t below = steps + 2, dc = (uint32_t)dt * pinv * J;
         uint32_t mul[J], c[J], thr[J];
         uint32_t power = 1;
 #pragma unroll
         for (int i = 0; i < J; ++i) {
             mul[i] = power * pinv;
-            c[i] = below - ((M - 1) * (uint32_t)(m + i) + M) * pinv;
+            c[i] = below - ((uint32_t)t + i * (uint32_t)dt) * pinv;
             thr[i] = below + 4 * power;
             power *= M;
         }
-        for (uint64_t g = 0; g < groups;) {
+        for (uint32_t g = 0; g < groups;) {
             uint64_t Y0;
             bool hit;
             do {
@@ -1728,7 +1731,7 @@ __device__ __noinline__ uint64_t smarandache_blocks64(const JobView &job, uint64
 #pragma unroll
                     for (int i = 0; i < J; ++i) {
                         cand |= lo * mul[i] + c[i] < thr[i];
-                        c[i] -= dt;
+                        c[i] -= dc;
                     }
                     uint32_t q;
                     if (J == 1)
@@ -1747,12 +1750,14 @@ __device__ __noinline__ uint64_t smarandache_blocks64(const JobView &job, uint64
                 hit = __any_sync(__activemask(), cand);
             } while (++g < groups && !hit);
             if (hit)
-                smarandache_exact64(job.fb, job.n0, p, Y0, M, Ms, m + (g - 1) * (GROUP * J), GROUP * J);
+                smarandache_exact64(job.fb, job.n0, p, Y0, t + (uint64_t)((g - 1) * (GROUP * J)) * dt, dt, M, Ms,
+                                    m + (g - 1) * (GROUP * J), GROUP * J);
         }
+        t += (uint64_t)(groups * (GROUP * J)) * dt;
         m += groups * (GROUP * J);
         steps -= groups * (GROUP * J);
     }
-    return smarandache_exact64(job.fb, job.n0, p, Y, M, Ms, m, (uint32_t)steps);
+    return smarandache_exact64(job.fb, job.n0, p, Y, t, dt, M, Ms, m, steps);
 }
 
 // Classes whose blocks take over from the walks of S: M up to 2^20 (J = 1's
@@ -1762,47 +1767,39 @@ __device__ __noinline__ uint64_t smarandache_blocks64(const JobView &job, uint64
 // SM_MIN_LAST would go by exact steps alone.
 constexpr uint64_t SM_MIN_CLASS = 2048, SM_MIN_LAST = 32;
 
-__device__ __forceinline__ void run_smarandache(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
+__device__ __forceinline__ bool smarandache_by_blocks(const JobView &job, uint64_t p, uint64_t pw, uint64_t mcur, uint64_t e)
+{
+    return (p >> 30) && !(p >> 44) && pw <= (1ull << 20) && e <= p && job.variant == CTD_VARIANT_AUTO &&
+           (pw >= e ? e - mcur >= SM_MIN_LAST : pw - mcur >= SM_MIN_CLASS);
+}
+
+// p >= 2^30 (or p < e).  The set-up's products are most of the work of a few
+// hundred terms, so below 2^40 they are narrow.
+template <class MT>
+__device__ __noinline__ void run_smarandache64(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
 {
     const uint64_t b = job.param;
     uint64_t mcur = s + 1;  // m = n + 1 of the next step
-    if (p < (1u << 30) && p >= e && e <= 0xffffffffull && job.variant != CTD_VARIANT_MONTGOMERY) {
-        // 32-bit words: x kept in [0, 3p) (Shoup output < 2p, plus D < p).
-        // The set-up in 32-bit Montgomery arithmetic
-        Mont32 m;
-        m.init(p);
-        uint32_t x = (uint32_t)m.from(smarandache_at(m, b, s));
-        while (mcur < e) {
-            uint64_t pw;
-            const uint64_t cend = class_end(b, mcur, pw);
-            const uint32_t M = (uint32_t)class_multiplier(m, b, mcur, pw);
-            const uint32_t first = (uint32_t)(mcur - 1), steps = (uint32_t)((cend < e ? cend : e) - mcur);
-            // J by the chance of a candidate, 4 M^(J-1) / 2^32 a block of each
-            // lane: at M = 1000 one in 1100 for J = 3 (an eighth of a warp's
-            // groups then step exactly, and the call took 7.2 ms for the 6.1
-            // that it takes with J = 2)
-            if (M <= 128)
-                x = smarandache_blocks32<3>(job, m, x, M, first, steps);
-            else if (M <= 1u << 20)
-                x = smarandache_blocks32<2>(job, m, x, M, first, steps);
-            else
-                x = smarandache_blocks32<1>(job, m, x, M, first, steps);
-            mcur += steps;
-        }
-        if (x == 0 || x == p || x == 2 * p)
-            push(job.fb, e - 1 - job.n0, p);
-        return;
-    }
-    Mont m;
+    MT m;
     m.init(p);
-    uint64_t X = smarandache_at(m, b, s);
+    // the class that holds s + 1 goes by blocks: S(s) is left a fraction
+    uint64_t X = 0, num = 0, den = m.one;
+    bool fraction = false;
+    if (s + 1 < e) {
+        uint64_t pw;
+        fraction = smarandache_by_blocks(job, p, class_end(b, s + 1, pw), s + 1, e);
+    }
+    if (fraction)
+        smarandache_fraction(m, b, s, num, den);
+    else
+        X = smarandache_at(m, b, s);
     if (p < (1ull << 62) && e <= p && job.variant != CTD_VARIANT_MONTGOMERY) {
         // every m < p.  A class goes by blocks of Y, by the Barrett-32 walk or
         // by the 64-bit Shoup walk; the walks keep x in [0, 3p) (x = 0 mod p
         // <=> x in {0, p, 2p}), test the low words only and replay a block
         // with a candidate with the full test.
         uint64_t x = m.from(X);
-        if (x == 0)
+        if (fraction ? num == 0 : x == 0)
             push(job.fb, s - job.n0, p);
         // Barrett-32 constants (p < 2^48): sh = floor(log2 p), mu = floor(2^(sh+32) / p)
         const uint32_t sh = 63 - clz64(p);
@@ -1817,29 +1814,31 @@ __device__ __forceinline__ void run_smarandache(const JobView &job, uint64_t p, 
             const uint64_t cend = class_end(b, mcur, pw);
             const uint64_t mend = cend < e ? cend : e;
             const uint64_t M = class_multiplier(m, b, mcur, pw);
-            if (sh >= 30 && sh < 52 && pw <= (1ull << 20) && job.variant == CTD_VARIANT_AUTO &&
-                mend - mcur >= (mend == e ? SM_MIN_LAST : SM_MIN_CLASS)) {
-                // (the states x = S(m) below 3p: to() reduces them)
-                const uint64_t a = m.to(M - 1), aa = m.mul(a, a);
-                const uint64_t Yf = m.add(m.mul(aa, m.to(x)), m.add(m.mul(a, m.to(mcur - 1)), m.to(M)));
-                uint64_t Y = m.from(Yf);
-                const uint32_t pinv = 0u - (uint32_t)m.pinv;
+            if (smarandache_by_blocks(job, p, pw, mcur, e)) {
+                // from S(mcur - 1) = num / den (x / 1, x below 3p, after the
+                // range's first class), which is tested: Y, times den, goes
+                // one term ahead
+                if (!fraction)
+                    num = m.to(x), den = m.one;
+                fraction = false;
+                // (an integer times a Montgomery form is the plain product)
+                const uint64_t aa = (M - 1) * (M - 1), dt = m.mul(M - 1, den);
+                const uint64_t t0 = m.mul((M - 1) * (mcur - 1) + M, den), t = m.add(t0, dt);
+                const uint32_t pinv = 0u - (uint32_t)m.pinv, steps = (uint32_t)(mend - mcur);
                 const uint64_t Ms = m.shoup(M);
-                // the class's terms are mcur .. mend - 1 (mcur - 1, the state
-                // it starts from, is tested): Y goes one term ahead
+                uint64_t Y = m.add(m.mul(aa, num), t0);
                 Y = Y * M - mulhi64(Y, Ms) * p;  // < 2p
                 if (M <= 812)
-                    Y = smarandache_blocks64<3>(job, p, pinv, Y, (uint32_t)M, Ms, m.shoup(M * M * M), mcur, mend - mcur);
+                    Y = smarandache_blocks64<3>(job, p, pinv, Y, t, dt, (uint32_t)M, Ms, m.shoup(M * M * M), mcur, steps);
                 else if (M <= 23170)
-                    Y = smarandache_blocks64<2>(job, p, pinv, Y, (uint32_t)M, Ms, m.shoup(M * M), mcur, mend - mcur);
+                    Y = smarandache_blocks64<2>(job, p, pinv, Y, t, dt, (uint32_t)M, Ms, m.shoup(M * M), mcur, steps);
                 else
-                    Y = smarandache_blocks64<1>(job, p, pinv, Y, (uint32_t)M, Ms, Ms, mcur, mend - mcur);
+                    Y = smarandache_blocks64<1>(job, p, pinv, Y, t, dt, (uint32_t)M, Ms, Ms, mcur, steps);
                 mcur = mend;
                 if (mend < e) {
-                    // Y = Y(mend): back one term to S(mend - 1) through
-                    // Y(mend) = M ((M-1)^2 S(mend-1) + t(mend-1))
-                    const uint64_t Mf = m.to(M), tf = m.add(m.mul(a, m.to(mend - 1)), Mf);
-                    const uint64_t inv = m.pow(m.mul(aa, Mf), p - 2);
+                    // back one term from Y(mend) = M ((M-1)^2 S(mend-1) + t(mend-1)) den
+                    const uint64_t tf = m.mul(m.to((M - 1) * (mend - 1) + M), den), Mf = m.to(M);
+                    const uint64_t inv = m.pow(m.mul(m.mul(m.to(aa), Mf), den), p - 2);
                     x = m.from(m.mul(m.sub(m.to(Y), m.mul(Mf, tf)), inv));
                 }
                 continue;
@@ -1875,6 +1874,43 @@ __device__ __forceinline__ void run_smarandache(const JobView &job, uint64_t p, 
                 push(job.fb, mcur - job.n0, p);
         }
     }
+}
+
+__device__ __forceinline__ void run_smarandache(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
+{
+    const uint64_t b = job.param;
+    uint64_t mcur = s + 1;  // m = n + 1 of the next step
+    if (p < (1u << 30) && p >= e && e <= 0xffffffffull && job.variant != CTD_VARIANT_MONTGOMERY) {
+        // 32-bit words: x kept in [0, 3p) (Shoup output < 2p, plus D < p).
+        // The set-up in 32-bit Montgomery arithmetic
+        Mont32 m;
+        m.init(p);
+        uint32_t x = (uint32_t)m.from(smarandache_at(m, b, s));
+        while (mcur < e) {
+            uint64_t pw;
+            const uint64_t cend = class_end(b, mcur, pw);
+            const uint32_t M = (uint32_t)class_multiplier(m, b, mcur, pw);
+            const uint32_t first = (uint32_t)(mcur - 1), steps = (uint32_t)((cend < e ? cend : e) - mcur);
+            // J by the chance of a candidate, 4 M^(J-1) / 2^32 a block of each
+            // lane: at M = 1000 one in 1100 for J = 3 (an eighth of a warp's
+            // groups then step exactly, and the call took 7.2 ms for the 6.1
+            // that it takes with J = 2)
+            if (M <= 128)
+                x = smarandache_blocks32<3>(job, m, x, M, first, steps);
+            else if (M <= 1u << 20)
+                x = smarandache_blocks32<2>(job, m, x, M, first, steps);
+            else
+                x = smarandache_blocks32<1>(job, m, x, M, first, steps);
+            mcur += steps;
+        }
+        if (x == 0 || x == p || x == 2 * p)
+            push(job.fb, e - 1 - job.n0, p);
+        return;
+    }
+    if (p < MONT_NARROW_LIMIT)
+        run_smarandache64<MontN>(job, p, s, e);
+    else
+        run_smarandache64<Mont>(job, p, s, e);
 }
 
 // Peano S(n) = n, the reference's engine test sequence (tests/peano.hpp).

@@ -190,4 +190,37 @@ CTD_HD uint64_t smarandache_at(const MT &m, uint64_t b, uint64_t s)
     return smarandache_at_closed(m, b, s);
 }
 
+// Sm_b(s) as a fraction N / Q mod p, both in Montgomery form (needs m.r2), for
+// s whose digit class ends at 2^20 at most.  Within the class of multiplier
+// M = b^d, Y(n) = (M-1)^2 Sm(n) + t(n), t(n) = (M-1) n + M, obeys Y(n+1) = M Y(n),
+// so a class of T terms after n takes N / Q to
+//   N' = M^T ((M-1)^2 N + t(n) Q) - t(n+T) Q,  Q' = (M-1)^2 Q:
+// five products and the power, no inverse.  The integers (M-1)^2 and t, below
+// 2^41, are multiplied as they are: that divides N' and Q' by R both.  The
+// powers of the whole classes come from one another: v(d) = b^((b-1) b^(d-1)),
+// M^T = v(d)^d, v(d+1) = v(d)^b.  p > b^d for every class (Q is then a unit).
+// At s = 20001 and base 7 about 90 products; the closed form takes 220.
+template <class MT>
+CTD_HD void smarandache_fraction(const MT &m, uint64_t b, uint64_t s, uint64_t &N, uint64_t &Q)
+{
+    N = 0;
+    Q = m.one;
+    const uint64_t bf = m.to(b);
+    uint64_t v = m.pow(bf, b - 1);
+    uint64_t lo = 1, M = b;  // the class of the d-digit n: lo .. M - 1
+    for (uint32_t d = 1; lo <= s; ++d) {
+        const bool whole = M - 1 <= s;
+        const uint64_t last = whole ? M - 1 : s;
+        const uint64_t P = whole ? m.pow(v, d) : m.pow(bf, d * (last - lo + 1));
+        const uint64_t aa = (M - 1) * (M - 1);
+        const uint64_t Y = m.add(m.mul(aa, N), m.mul((M - 1) * (lo - 1) + M, Q));
+        N = m.sub(m.mul(P, Y), m.mul((M - 1) * last + M, Q));
+        Q = m.mul(aa, Q);
+        if (whole)
+            v = m.pow(v, b);
+        lo = M;
+        M *= b;
+    }
+}
+
 }  // namespace ctd
