@@ -362,19 +362,27 @@ struct TargetFilter {
 
     __device__ __forceinline__ uint2 &slot(uint32_t h) const { return col[(h >> 27) * stride]; }
 
-    // marks the 32 targets' low words
-    __device__ __forceinline__ void build(const uint32_t (&tlo)[BS]) const
+    __device__ __forceinline__ void clear() const
     {
 #pragma unroll 8
         for (int k = 0; k < FILTER_SLOTS; ++k)
             col[k * stride] = uint2{0, 0};
+    }
+    // marks a target's low word
+    __device__ __forceinline__ void insert(uint32_t t) const
+    {
+        const uint32_t h = t * FILTER_A;
+        uint2 &sl = slot(h);
+        sl.x |= 1u << (t & 31);
+        sl.y |= 1u << ((h >> 22) & 31);
+    }
+    // marks the 32 targets' low words
+    __device__ __forceinline__ void build(const uint32_t (&tlo)[BS]) const
+    {
+        clear();
 #pragma unroll 4
-        for (int j = 0; j < BS; ++j) {
-            const uint32_t t = tlo[j], h = t * FILTER_A;
-            uint2 &sl = slot(h);
-            sl.x |= 1u << (t & 31);
-            sl.y |= 1u << ((h >> 22) & 31);
-        }
+        for (int j = 0; j < BS; ++j)
+            insert(tlo[j]);
     }
 
     // bit 0 set if lo may equal one of the targets (always when it does);
@@ -639,9 +647,6 @@ __device__ __forceinline__ uint64_t doubling_target_of(const JobView &job, uint6
                                   : doubling_target<MERSENNE>(job, p);
 }
 
-// The doubling walk over n = r (mod M) in [s, e), p < 2^63.  One body for
-// the three families (they differ only in the target), so the kernels that
-// walk classes of several families hold one copy of it.
 // 2^-x in Montgomery form: left-to-right powering of 2^-1, each set bit a
 // halving of the Montgomery representative ((x R) / 2 = (x / 2) R) -- as many
 // squarings as x has bits
@@ -666,6 +671,72 @@ __device__ __forceinline__ uint64_t div_small(uint64_t x, uint32_t M)
     return x >> 32 ? x / M : (uint32_t)x / M;
 }
 
+// 2^-M in Montgomery form, one = R mod p: a partial reduction while M < 64
+__device__ __forceinline__ uint64_t half_form(const Mont &m, uint32_t M)
+{
+    if (M >= 64)
+        return pow_half(m, M);
+    const uint64_t mm = m.one * m.pinv & ((1ull << M) - 1);
+    const uint64_t lo = m.one + mm * m.p, hi = mulhi64(mm, m.p) + (lo < m.one);
+    return M ? (hi << (64 - M)) | (lo >> M) : lo;
+}
+
+// Blocks of a class, B = 32 or 64 terms, from x = w(first term): a block's
+// state is w one term past its end, giant(x), and term j of it is a zero iff
+// that equals wt 2^(-M (B - j)) -- the targets need no other constant than the
+// step to the next term, 2^-M.  tlo holds the low words of all targets (B =
+// 32), or of every second one, i = 2, 4, .., 64 (B = 64: a state meets an odd
+// target iff the state times 2^-M meets the next even one); the filter holds
+// them all.  ng groups share a vote each; replay(z, b) settles block b of state
+// z.  Terms past the range's end are left to replay.
+//
+// Twice the targets in the same filter pass 3 times the states (0.6 %), so a
+// warp's block takes the exact compares every sixth time instead of every
+// sixteenth, but there are half the giant steps, tests and votes: worth the 32
+// more targets (some 900 instructions) from CLASS_LONG terms.
+constexpr uint64_t CLASS_LONG = 2560;
+template <int B, class Giant, class Near, class Replay>
+__device__ __forceinline__ void class_blocks(const TargetFilter &flt, const uint32_t (&tlo)[BS], uint64_t x, uint32_t ng,
+                                             Giant giant, Near near, Replay replay)
+{
+    constexpr int G = B == 64 ? 2 : FILTER_GROUP;
+    for (uint32_t g = 0; g < ng; ++g) {
+        const uint64_t x0 = x;
+        uint32_t fs[G], any = 0;
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+            x = giant(x);
+            fs[i] = flt.test((uint32_t)x) & 1;
+            any |= fs[i];
+        }
+        if (__any_sync(__activemask(), any)) {
+            const uint32_t act = __activemask();
+            uint32_t pass = 0;
+#pragma unroll
+            for (int i = 0; i < G; ++i)
+                pass |= fs[i] << i;
+            uint64_t z = x0;
+            int at = -1;
+            for (uint32_t todo = __reduce_or_sync(act, pass); todo; todo &= todo - 1) {
+                const int i = __ffs(todo) - 1;
+                for (; at < i; ++at)
+                    z = giant(z);
+                uint32_t cand = 0;
+                if ((pass >> i) & 1) {
+                    cand = match32((uint32_t)z, tlo);
+                    if (B == 64)
+                        cand |= match32((uint32_t)near(z), tlo);
+                }
+                if (__any_sync(act, cand))
+                    replay(z, (uint64_t)g * G + i);
+            }
+        }
+    }
+}
+
+// The doubling walk over n = r (mod M) in [s, e), p < 2^63.  One body for
+// the three families (they differ only in the target), so the kernels that
+// walk classes of several families hold one copy of it.
 __device__ void run_doubling_class(const JobView &job, uint64_t p, uint32_t M, uint32_t r, uint64_t s, uint64_t e)
 {
     const uint32_t sr = mod_small(s, M);
@@ -681,55 +752,76 @@ __device__ void run_doubling_class(const JobView &job, uint64_t p, uint32_t M, u
     m.init_lite(p);
     const uint64_t wt = doubling_target_of(job, p);
     const uint64_t nr = nf < p - 1 ? nf : nf % (p - 1);
-    uint64_t w = m.from(pow_half(m, nr));  // 2^-nf
-    const uint64_t HM = pow_half(m, M);    // 2^-M in Montgomery form
-    const MulConst step{m.from(HM), HM * m.pinv};  // w -> w 2^-M: the next term of the class
+    uint64_t w = half_power<false>(p, m.pinv, nr);  // 2^-nf
+    const uint64_t HM = half_form(m, M);            // 2^-M in Montgomery form
+    const MulConst step{m.from(HM), HM * m.pinv};   // w -> w 2^-M: the next term of the class
     const uint64_t at0 = nf - job.n0;
-    uint64_t i = 0;
-    if (cnt >= 2 * BS) {
-        // targets wt 2^(M j), j < 32: term j of a block is a zero iff the
-        // block's state equals target j
-        const uint64_t C = m.pow2(M);
-        const MulConst up{m.from(C), C * m.pinv};
-        uint32_t tlo[BS];
-        uint64_t t = wt;
+    if (cnt < 2 * BS) {  // term by term
+        for (uint64_t i = 0; i < cnt; ++i) {
+            if (w == wt)
+                push_call(job.fb, at0 + i * M, p);
+            w = step.mul(w, p);
+        }
+        return;
+    }
+    const TargetFilter flt;
+    uint32_t tlo[BS];
+    uint64_t t = wt;
+    // the exact test of a block: its state against the targets, last term first
+    auto replay = [&](uint64_t z, uint64_t first, int terms) {
+        uint64_t v = wt;
+#pragma unroll 1
+        for (int i = 1; i <= terms; ++i) {
+            v = step.mul(v, p);
+            const uint64_t term = first + (uint64_t)(terms - i);
+            if (z == v && term < cnt)
+                push_call(job.fb, at0 + term * M, p);
+        }
+    };
+    auto near = [&](uint64_t x) { return step.mul(x, p); };
+    const uint32_t plo = (uint32_t)p, phi = (uint32_t)(p >> 32), pinv32 = (uint32_t)m.pinv, one = (uint32_t)(p & 1);
+    auto redc = [&](uint64_t x) { return redc32(x, plo, phi, pinv32, one); };
+    // (the warp's lanes walk classes of about the same M: one block length)
+    if (__any_sync(__activemask(), cnt >= CLASS_LONG)) {
+        flt.clear();
 #pragma unroll
         for (int j = 0; j < BS; ++j) {
+            t = step.mul(t, p);
+            flt.insert((uint32_t)t);
+            t = step.mul(t, p);
+            flt.insert((uint32_t)t);
             tlo[j] = (uint32_t)t;
-            t = up.mul(t, p);
         }
-        auto replay = [&](uint64_t v, uint64_t b) {
-#pragma unroll 1
-            for (int j = 0; j < BS; ++j) {
-                if (v == wt)
-                    push_call(job.fb, at0 + (b * BS + j) * M, p);
-                v = step.mul(v, p);
-            }
-        };
-        const uint64_t nb = cnt / BS;
-        if (M <= 2) {
-            // giant step w 2^-32M: one or two 32-bit Montgomery reductions
-            // (a loop of M reductions for M up to 4, measured, ran the walk
-            // 34 % slower than the 64-bit Shoup product for M = 3, 4)
-            const uint32_t plo = (uint32_t)p, phi = (uint32_t)(p >> 32), pinv32 = (uint32_t)m.pinv;
-            const uint32_t one = (uint32_t)(p & 1);
-            if (M == 1)
-                w = run_blocks(tlo, w, nb, [&](uint64_t x) { return redc32(x, plo, phi, pinv32, one); }, replay);
-            else
-                w = run_blocks(tlo, w, nb,
-                               [&](uint64_t x) { return redc32(redc32(x, plo, phi, pinv32, one), plo, phi, pinv32, one); },
-                               replay);
+        const uint32_t ng = (uint32_t)((cnt + 127) / 128);
+        auto long_replay = [&](uint64_t z, uint64_t b) { replay(z, b * 64, 64); };
+        if (M == 1) {
+            class_blocks<64>(flt, tlo, w, ng, [&](uint64_t x) { return redc(redc(x)); }, near, long_replay);
         } else {
-            const uint64_t G = square_n(m, HM, 5);  // 2^-32M in Montgomery form
-            const MulConst giant{m.from(G), G * m.pinv};
-            w = run_blocks(tlo, w, nb, [&](uint64_t x) { return giant.mul(x, p); }, replay);
+            const uint64_t Gf = square_n(m, HM, 6);  // 2^-64M in Montgomery form
+            const MulConst giant{m.from(Gf), Gf * m.pinv};
+            class_blocks<64>(flt, tlo, w, ng, [&](uint64_t x) { return giant.mul(x, p); }, near, long_replay);
         }
-        i = nb * BS;
+        return;
     }
-    for (; i < cnt; ++i) {  // the tail, term by term
-        if (w == wt)
-            push_call(job.fb, at0 + i * M, p);
-        w = step.mul(w, p);
+#pragma unroll
+    for (int j = 0; j < BS; ++j) {
+        t = step.mul(t, p);
+        tlo[j] = (uint32_t)t;
+    }
+    const uint64_t Gf = square_n(m, HM, 5);  // 2^-32M in Montgomery form
+    const MulConst giant{m.from(Gf), Gf * m.pinv};
+    auto far = [&](uint64_t x) { return giant.mul(x, p); };
+    const uint32_t nb = (uint32_t)((cnt + BS - 1) / BS);
+    if (nb >= FILTER_MIN_BLOCKS) {
+        flt.build(tlo);
+        class_blocks<32>(flt, tlo, w, (nb + FILTER_GROUP - 1) / FILTER_GROUP, far, near,
+                         [&](uint64_t z, uint64_t b) { replay(z, b * BS, BS); });
+    } else {
+        for (uint32_t b = 0; b < nb; ++b) {
+            w = far(w);
+            if (match32((uint32_t)w, tlo))
+                replay(w, (uint64_t)b * BS, BS);
+        }
     }
 }
 
