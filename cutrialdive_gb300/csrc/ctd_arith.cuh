@@ -249,12 +249,20 @@ struct MontT {
         return r;
     }
 };
-// 2^-x mod p for odd p (NARROW: p < 2^40), pinv = -p^-1 mod 2^64.  2^-f is (1 + m p) / 2^f
-// with m = pinv mod 2^f, for f below 64 at once; with X(e) = 2^(64-e) mod p the
-// Montgomery product of X(a) and X(b) is X(a+b), halving X(e) gives X(e+1), and
-// X(64+f) = 2^-f: the seven leading bits of a longer x cost that one product,
-// each further bit a squaring, and nothing needs R mod p, a 64-bit division.
-// (2^(p-1-x) by Fermat takes a squaring for every bit of p.)
+// 2^-f mod p for odd p, f < 64, pinv = -p^-1 mod 2^64: (1 + m p) / 2^f with
+// m = pinv mod 2^f.  It is also 2^-(64+f) in Montgomery form.
+CTD_HD uint64_t half_power_start(uint64_t p, uint64_t pinv, uint32_t f)
+{
+    const uint64_t mm = pinv & ((1ull << f) - 1);
+    const uint64_t lo = mm * p + 1, hi = mulhi64(mm, p) + (lo == 0);
+    return f ? (hi << (64 - f)) | (lo >> f) : lo;
+}
+
+// 2^-x mod p for odd p (NARROW: p < 2^40), pinv = -p^-1 mod 2^64.  With X(e) =
+// 2^(64-e) mod p the Montgomery product of X(a) and X(b) is X(a+b), halving X(e)
+// gives X(e+1), and X(64+f) = 2^-f: the seven leading bits of a longer x cost
+// that one product, each further bit a squaring, and nothing needs R mod p, a
+// 64-bit division.  (2^(p-1-x) by Fermat takes a squaring for every bit of p.)
 template <bool NARROW>
 CTD_HD uint64_t half_power(uint64_t p, uint64_t pinv, uint64_t x)
 {
@@ -263,10 +271,7 @@ CTD_HD uint64_t half_power(uint64_t p, uint64_t pinv, uint64_t x)
     m.pinv = pinv;
     const int bits = 64 - clz64(x | 64);       // 7 and more
     const int rest = x < 64 ? 0 : bits - 7;    // bits of x after the leading ones
-    const uint32_t f = (uint32_t)(x >> rest) & 63;
-    const uint64_t mask = (1ull << f) - 1, mm = pinv & mask;
-    const uint64_t lo = mm * p + 1, hi = mulhi64(mm, p) + (lo == 0);
-    uint64_t r = f ? (hi << (64 - f)) | (lo >> f) : lo;
+    uint64_t r = half_power_start(p, pinv, (uint32_t)(x >> rest) & 63);
     if (x < 64)
         return r;
     for (int b = rest - 1; b >= 0; --b) {

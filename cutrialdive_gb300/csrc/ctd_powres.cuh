@@ -206,29 +206,69 @@ CTD_HD bool quadratic_excluded(uint64_t p, uint64_t k, bool negate)
 // in one left-to-right loop over the bits of e: per bit a squaring of each,
 // and for a set bit a halving of A's Montgomery representative ((x R)/2 =
 // (x/2) R) and a Shoup multiplication of B by the plain k -- two
-// independent chains per iteration.  0 < e < p - 1, p < 2^63 (m needs no r2).
+// independent chains per iteration.  A takes the seven leading bits of e at
+// once (half_power_start).  0 < e < p - 1, p < 2^63 (m needs no r2).
 template <class MT>
 CTD_HD void power_pair(const MT &m, uint64_t k, bool negate, uint64_t e, uint64_t &A, uint64_t &B)
 {
     const uint64_t p = m.p;
     const uint64_t kr = k < p ? k : k % p;
     const uint64_t ks = m.shoup_any(kr);
-    A = m.one;
-    B = m.one;
+    int b = 63 - clz64(e);
+    B = shoup_mul(m.one, kr, ks, p);  // the leading bit
     // A and B stay below 2p (the narrow product's lazy form; a halving of
     // x < 2p is below 1.5p; Shoup's product of x < 2^64 is below p)
-    for (int b = 63 - clz64(e); b >= 0; --b) {
-        A = m.mul_lazy(A, A);  // inline: the hot loop stays small
+    auto step_b = [&]() {
         B = m.mul_lazy(B, B);
-        if ((e >> b) & 1) {
-            A = (A + ((A & 1) ? p : 0)) >> 1;
+        if ((e >> b) & 1)
             B = shoup_mul(B, kr, ks, p);
+    };
+    if (b >= 6) {
+        const int rest = b - 6;
+        A = half_power_start(p, m.pinv, (uint32_t)(e >> rest) & 63);
+        for (--b; b >= rest; --b)
+            step_b();
+    } else {
+        A = m.one;
+        A = (A + ((A & 1) ? p : 0)) >> 1;
+        --b;
+        for (int a = b; a >= 0; --a) {
+            A = m.mul_lazy(A, A);
+            if ((e >> a) & 1)
+                A = (A + ((A & 1) ? p : 0)) >> 1;
         }
+        for (; b >= 0; --b)
+            step_b();
+    }
+    for (; b >= 0; --b) {
+        A = m.mul_lazy(A, A);  // inline: the hot loop stays small
+        if ((e >> b) & 1)
+            A = (A + ((A & 1) ? p : 0)) >> 1;
+        step_b();
     }
     A = m.canon(A);
     B = m.canon(B);
     if (negate && (e & 1))
         B = B ? p - B : 0;
+}
+
+// The 2-power condition from z = 2^-e and y = wt^e, e = (p - 1) / 2^u times a
+// unit, u = min(3, v) with 2^v the power of 2 in p - 1: n mod the order of z
+// into c, or false when y lies outside <z> (no zero at all).  The order of z is
+// 1, 2 or 4: for v <= 2 it divides 2^v, and where 8 | p - 1, 2 is a square, so
+// z^4 = 1 again.  z^2 = -1 when the order is 4, and y is one of 1, z, -1, -z:
+// three products (a scan of the eighth roots of unity took thirteen).
+template <class MT>
+CTD_HD bool two_part(const MT &m, uint64_t z, uint64_t y, PowerClass &c)
+{
+    auto mul = [&](uint64_t a, uint64_t b) { return powres_mul<MT>(a, b, m.p, m.pinv); };
+    const uint64_t z2 = mul(z, z), y2 = mul(y, y), y4 = mul(y2, y2);
+    const bool one = z == m.one, two = z2 == m.one;
+    if ((one ? y : two ? y2 : y4) != m.one)
+        return false;
+    c.M = one ? 1 : two ? 2 : 4;
+    c.r = y == m.one ? 0 : y == z ? 1 : y == z2 ? 2 : 3;
+    return true;
 }
 
 // The class of the zeros of 2^-n = wt (mod p), wt = -k (negate) or k, for
@@ -261,50 +301,21 @@ CTD_HD PowerClass doubling_class(const MT &m, uint64_t k, bool negate)
     // that does, they differ from (p - 1)/q by a factor prime to q, which
     // changes neither the order of z nor the logarithm j of y = z^j.
     PowerClass c{1, 0};
-    // ---- the 2-power part: z = A^105 of order 2^i (i <= u)
+    // ---- the 2-power part: z = A^105
     const Pow105 pa = pow105(m, A), pb = pow105(m, B);
     {
         const uint64_t z = pa.p105, y = pb.p105;
-        uint64_t zs = z, ys = y;
-        int i = 0;
-        bool y_ok = ys == m.one;
-        bool found = zs == m.one;
-#pragma unroll
-        for (int t = 1; t <= POWRES_MAX_2EXP; ++t) {
-            zs = mul(zs, zs);
-            ys = mul(ys, ys);
-            if (!found && t <= u) {
-                i = t;
-                y_ok = ys == m.one;
-                found = zs == m.one;
-            }
-        }
-        if (!y_ok)
-            return PowerClass{0, 0};  // y outside <z>: no zero at all
-        // the logarithm j < 2^i of y to the base z, by a scan of z^j
-        uint32_t j = 0;
-        uint64_t t = m.one;
-#pragma unroll
-        for (uint32_t jj = 0; jj < (1u << POWRES_MAX_2EXP); ++jj) {
-            if (jj < (1u << i) && t == y)
-                j = jj;
-            if (jj + 1 < (1u << POWRES_MAX_2EXP))
-                t = mul(t, z);
-        }
-        c.M = 1u << i;
-        c.r = j;
+        if (!two_part(m, z, y, c))
+            return PowerClass{0, 0};
     }
-    // ---- q = 3, 5, 7: z = A^(2^u 105 / q) = (A^(105/q))^(2^u), squarings
-    // of the chain's values (a loop of fixed length)
+    // ---- q = 3, 5, 7: z = A^(4 105 / q), y alike (the 2-parts of both have
+    // an order of 4 at most, as the 2-power part found)
     uint64_t zq[3] = {pa.p35, pa.p21, pa.p15}, yq[3] = {pb.p35, pb.p21, pb.p15};
 #pragma unroll
-    for (int t = 0; t < POWRES_MAX_2EXP; ++t)
-#pragma unroll
-        for (int kq = 0; kq < 3; ++kq) {
-            const uint64_t z2 = mul(zq[kq], zq[kq]), y2 = mul(yq[kq], yq[kq]);
-            zq[kq] = t < u ? z2 : zq[kq];
-            yq[kq] = t < u ? y2 : yq[kq];
-        }
+    for (int kq = 0; kq < 3; ++kq) {
+        zq[kq] = mul(zq[kq], zq[kq]), yq[kq] = mul(yq[kq], yq[kq]);
+        zq[kq] = mul(zq[kq], zq[kq]), yq[kq] = mul(yq[kq], yq[kq]);
+    }
     const uint32_t qs[3] = {3, 5, 7};
 #pragma unroll
     for (int kq = 0; kq < 3; ++kq) {
@@ -411,38 +422,13 @@ CTD_HD PowerClass doubling_class_pat(const MT &m, uint64_t k, bool negate)
     odd_powers<PAT>(m, A, ad, aq);
     odd_powers<PAT>(m, B, bd, bq);
     PowerClass c{1, 0};
-    // ---- the 2-power part: z = A^D_odd of order 2^i (i <= u)
+    // ---- the 2-power part: z = A^D_odd
     {
         const uint64_t z = ad, y = bd;
-        uint64_t zs = z, ys = y;
-        int i = 0;
-        bool y_ok = ys == m.one;
-        bool found = zs == m.one;
-#pragma unroll
-        for (int t = 1; t <= POWRES_MAX_2EXP; ++t) {
-            zs = mul(zs, zs);
-            ys = mul(ys, ys);
-            if (!found && t <= u) {
-                i = t;
-                y_ok = ys == m.one;
-                found = zs == m.one;
-            }
-        }
-        if (!y_ok)
+        if (!two_part(m, z, y, c))
             return PowerClass{0, 0};
-        uint32_t j = 0;
-        uint64_t t = m.one;
-#pragma unroll
-        for (uint32_t jj = 0; jj < (1u << POWRES_MAX_2EXP); ++jj) {
-            if (jj < (1u << i) && t == y)
-                j = jj;
-            if (jj + 1 < (1u << POWRES_MAX_2EXP))
-                t = mul(t, z);
-        }
-        c.M = 1u << i;
-        c.r = j;
     }
-    // ---- the q of PAT: z = (A^(D_odd/q))^(2^u)
+    // ---- the q of PAT: z = A^(4 D_odd / q), y alike (as in doubling_class)
     const uint32_t qs[3] = {3, 5, 7};
 #pragma unroll
     for (int kq = 0; kq < 3; ++kq) {
@@ -450,12 +436,8 @@ CTD_HD PowerClass doubling_class_pat(const MT &m, uint64_t k, bool negate)
             continue;
         const uint32_t q = qs[kq];
         uint64_t z = aq[kq], y = bq[kq];
-#pragma unroll
-        for (int t = 0; t < POWRES_MAX_2EXP; ++t) {
-            const uint64_t z2 = mul(z, z), y2 = mul(y, y);
-            z = t < u ? z2 : z;
-            y = t < u ? y2 : y;
-        }
+        z = mul(z, z), y = mul(y, y);
+        z = mul(z, z), y = mul(y, y);
         if (z == m.one) {
             if (y != m.one)
                 return PowerClass{0, 0};
