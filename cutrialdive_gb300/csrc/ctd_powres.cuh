@@ -83,20 +83,6 @@ inline uint64_t powres_mul(uint64_t a, uint64_t b, uint64_t p, uint64_t pinv)
 }
 #endif
 
-// base^e (base in Montgomery form, e small)
-template <class MT>
-CTD_HD uint64_t small_pow(const MT &m, uint64_t base, uint32_t e)
-{
-    uint64_t r = m.one;
-    while (e) {
-        if (e & 1)
-            r = m.mul(r, base);
-        base = m.mul(base, base);
-        e >>= 1;
-    }
-    return r;
-}
-
 // x^(2^s)
 template <class MT>
 CTD_HD uint64_t square_n(const MT &m, uint64_t x, int s)
@@ -504,8 +490,9 @@ CTD_HD uint32_t rare_q_of(uint64_t p, uint32_t qmax)
     return found;
 }
 
-// j < q with z^j = y, for z of prime order q, 11 <= q <= 127 (baby steps
-// z^0 .. z^7, giant steps by z^-8 = z^(q - 8)); q when there is none
+// j < q with z^j = y, for z of prime order q, 11 <= q <= 127; q when there is
+// none: baby steps z^0 .. z^7, giant steps y z^8i, so that j = b - 8 i mod q
+// where one meets the other (with steps y z^-8i, z^(q-8) took 13 products more)
 template <class MT>
 CTD_HD uint32_t small_log(const MT &m, uint64_t z, uint64_t y, uint32_t q)
 {
@@ -515,14 +502,14 @@ CTD_HD uint32_t small_log(const MT &m, uint64_t z, uint64_t y, uint32_t q)
 #pragma unroll
     for (int j = 1; j < 8; ++j)
         baby[j] = mul(baby[j - 1], z);
-    const uint64_t g = small_pow(m, z, q - 8);
+    const uint64_t g = mul(baby[7], z);
     uint64_t t = y;
     uint32_t found = q;
     for (uint32_t i = 0; 8 * i < q && found == q; ++i) {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            if (t == baby[j] && 8 * i + j < q && found == q)
-                found = 8 * i + j;
+            if (t == baby[j])
+                found = (uint32_t)j >= 8 * i ? j - 8 * i : j + q - 8 * i;
         t = mul(t, g);
     }
     return found;
@@ -540,7 +527,8 @@ CTD_HD PowerClass refine_class(const MT &m, uint64_t k, bool negate, PowerClass 
     if (!c.M || !q)
         return c;
     uint64_t z, y;
-    power_pair(m, k, negate, (m.p - 1) / q, z, y);
+    // (p - 1) / q is exact: a product with q^-1 mod 2^64
+    power_pair(m, k, negate, (m.p - 1) * ((uint64_t)0 - MT::neg_inverse(q)), z, y);
     if (z == m.one)
         return y == m.one ? c : PowerClass{0, 0};
     const uint32_t j = small_log(m, z, y, q);
