@@ -288,12 +288,43 @@ void tiles_for(uint64_t nprimes, uint64_t N, int grid, int block, uint32_t items
     tiles = (uint32_t)((N + tile_len - 1) / tile_len);
 }
 
+// Shortest index tile of a list that leaves the GPU's threads idle, in terms:
+// about the terms that a tile's start costs (2^-n for the doubling families,
+// whose shortest block is 32 terms; a jump of thousands of instructions for
+// the others).  0: the family's work does not grow with the terms.  The 11,000
+// primes of a 2^18-wide range at 2^33 or 2^34: Proth, 2000 terms, 282 us in one
+// tile and 110 in shorter ones; Smarandache, 4000 terms, 533 and 208;
+// tribonacci, 50,000 terms, 1176 in tiles of 4096 terms and 286 (both with the
+// step's other changes).
+uint32_t short_list_tile(uint32_t family)
+{
+    switch (family) {
+    case CTD_PROTH:
+    case CTD_RIESEL:
+    case CTD_MERSENNE: return 40;
+    case CTD_PROTH_FIXED_N:
+    case CTD_RIESEL_FIXED_N: return 0;
+    default: return 512;
+    }
+}
+
 void choose_tiles(const ctd_ctx *ctx, uint32_t family, int bits, uint64_t nprimes, uint64_t N, int grid, int block,
                   uint32_t &tiles, uint64_t &tile_len)
 {
     const ctd_tuning *t = tuning_of(ctx, family, bits);
     tiles_for(nprimes, N, grid, block, t && t->items_per_thread ? t->items_per_thread : DEFAULT_ITEMS_PER_THREAD,
               t && t->min_tile ? t->min_tile : DEFAULT_MIN_TILE, tiles, tile_len);
+    // fewer items than threads: shorter tiles, until each thread has one
+    const uint64_t threads = (uint64_t)grid * block;
+    const uint32_t shortest = short_list_tile(family);
+    if (!t && shortest && nprimes * tiles < threads && N >= 2 * (uint64_t)shortest) {
+        uint64_t n = nprimes ? threads / nprimes : 1;
+        n = n < N / shortest ? n : N / shortest;
+        if (n > tiles) {
+            tile_len = (N + n - 1) / n;
+            tiles = (uint32_t)((N + tile_len - 1) / tile_len);
+        }
+    }
 }
 
 uint32_t variant_of(const ctd_ctx *ctx, uint32_t family, int bits)

@@ -154,7 +154,7 @@ __device__ __noinline__ uint64_t rank_of(uint64_t p, uint64_t S, uint32_t q1, ui
 }
 
 // The hits of the lanes' primes (those with mine; the whole warp calls):
-// n = a, 2a, ... or a/2, 3a/2, ..., each lane's in turn over the warp.
+// n = a, 2a, ... or a/2, 3a/2, ...
 template <uint32_t FAM, bool NARROW>
 __device__ __noinline__ void rank_push(const JobView &job, bool mine, uint64_t p, uint64_t S, unsigned long long top)
 {
@@ -165,14 +165,23 @@ __device__ __noinline__ void rank_push(const JobView &job, bool mine, uint64_t p
         a = p == 5 ? 5 : rank_of<NARROW>(p, S, (uint32_t)(top >> 32), (uint32_t)top, amax);
     if (a > amax || (FAM == LUCAS && (a & 1)))
         a = 0;
+    // first hit n = h mod a, and how many
+    uint64_t first = 0, hits = 0;
+    if (a) {
+        const uint64_t h = FAM == FIBONACCI ? 0 : a >> 1, r = s % a;
+        first = s + (h >= r ? h - r : a - r + h);
+        hits = first < e ? (e - 1 - first) / a + 1 : 0;
+    }
+    // few hits: every lane pushes its own; many: the warp a lane's together
     const uint32_t lane = threadIdx.x & 31u;
+    if (hits <= 8)
+        for (uint64_t i = 0; i < hits; ++i)
+            push(job.fb, first + i * a - s, p);
     __syncwarp();
-    for (uint32_t todo = __ballot_sync(0xffffffffu, a != 0); todo; todo &= todo - 1) {
-        const uint64_t pk = __shfl_sync(0xffffffffu, p, __ffs(todo) - 1), ak = __shfl_sync(0xffffffffu, a, __ffs(todo) - 1);
-        const uint64_t h = FAM == FIBONACCI ? 0 : ak >> 1;
-        const uint64_t r = s % ak;
-        const uint64_t first = s + (h >= r ? h - r : ak - r + h);
-        for (uint64_t x = first + lane * ak; x < e; x += 32 * ak)
+    for (uint32_t todo = __ballot_sync(0xffffffffu, hits > 8); todo; todo &= todo - 1) {
+        const int from = __ffs(todo) - 1;
+        const uint64_t pk = __shfl_sync(0xffffffffu, p, from), ak = __shfl_sync(0xffffffffu, a, from);
+        for (uint64_t x = __shfl_sync(0xffffffffu, first, from) + lane * ak; x < e; x += 32 * ak)
             push(job.fb, x - s, pk);
         __syncwarp();
     }
@@ -511,7 +520,7 @@ rank_kernel(JobView job, const uint64_t *__restrict__ primes, uint64_t nprimes, 
         if (!rank_tile<FAM>(job, list, sh, primes + first, n, nq)) {
             // a sparse or unordered stretch of the list: item by item
             for (uint64_t k = threadIdx.x; k < (uint64_t)n * job.tiles; k += 256)
-                residue_item<FAM>(job, primes + first, k);
+                residue_item<FAM>(job, primes + first, n, k);
         }
     }
 }

@@ -38,9 +38,10 @@ uint64_t kernel_launch_count() { return g_launches.load(std::memory_order_relaxe
 // Keeps a term's max_factors smallest primes once more primes than slots
 // divide it.  Called together by the lanes `peers` pushing to the same
 // term; `pending` lanes still hold a prime without a slot.  Each round the
-// leader finds the largest value in the slots (an empty slot, 0, counts as
-// larger than any prime); every pending lane whose prime is not below it
-// gives up (values only decrease, so it never will be), and the lowest
+// lanes find the largest value in the slots, a share of them each (an empty
+// slot, 0, counts as larger than any prime; one lane reading all 32 made a
+// call whose primes all divide T(1) five times as long); every pending lane
+// whose prime is not below it gives up (values only decrease, so it never will be), and the lowest
 // remaining lane replaces that value with its prime by an exchange.  Each
 // successful exchange replaces the current largest value by a smaller one,
 // so after all pushes the slots hold the smallest primes pushed, whatever
@@ -48,36 +49,39 @@ uint64_t kernel_launch_count() { return g_launches.load(std::memory_order_relaxe
 // primes in ascending order.  A failed exchange (another push changed the
 // slots) leaves the lane pending; the rounds are bounded.
 __device__ __forceinline__ void push_overflow(unsigned long long *slots, uint32_t k, unsigned long long p, bool pending,
-                                           uint32_t peers, int leader)
+                                              uint32_t peers)
 {
-    const int lane = (int)(threadIdx.x & 31u);
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t rank = __popc(peers & ((1u << lane) - 1u)), lanes = __popc(peers);
     for (int round = 0; round < (1 << 16); ++round) {
         if (!__any_sync(peers, pending))
             return;
-        unsigned long long m = 0, raw = 0;
+        // the lanes share the slots.  Volatile loads: another SM's exchanges
+        // must show (the exchange below checks what they read); an empty slot
+        // ends a lane's share
+        unsigned long long key = 0, raw = 0;
         uint32_t j = 0;
-        if (lane == leader) {
-            // volatile loads: another SM's exchanges must show (the
-            // exchange below checks what they read); an empty slot ends it
-            for (uint32_t i = 0; i < k; ++i) {
-                const unsigned long long v = *(volatile unsigned long long *)&slots[i];
-                const unsigned long long key = v ? v : ~0ull;
-                if (key > m) {
-                    m = key;
-                    raw = v;
-                    j = i;
-                    if (!v)
-                        break;
-                }
+        for (uint32_t i = rank; i < k; i += lanes) {
+            const unsigned long long v = *(volatile unsigned long long *)&slots[i];
+            const unsigned long long x = v ? v : ~0ull;
+            if (x > key) {
+                key = x;
+                raw = v;
+                j = i;
+                if (!v)
+                    break;
             }
         }
-        m = __shfl_sync(peers, m, leader);
-        raw = __shfl_sync(peers, raw, leader);
-        j = __shfl_sync(peers, j, leader);
+        const uint32_t high = __reduce_max_sync(peers, (uint32_t)(key >> 32));
+        const uint32_t low = __reduce_max_sync(peers, key >> 32 == high ? (uint32_t)key : 0u);
+        const unsigned long long m = (unsigned long long)high << 32 | low;
+        const int owner = __ffs(__ballot_sync(peers, key == m)) - 1;
+        raw = __shfl_sync(peers, raw, owner);
+        j = __shfl_sync(peers, j, owner);
         if (pending && p >= m)
             pending = false;
         const uint32_t want = __ballot_sync(peers, pending);
-        if (want && lane == __ffs(want) - 1 && atomicCAS(&slots[j], raw, p) == raw)
+        if (want && lane == (uint32_t)__ffs(want) - 1 && atomicCAS(&slots[j], raw, p) == raw)
             pending = false;
     }
 }
@@ -109,7 +113,7 @@ __device__ __forceinline__ void push(const FactorsView &fb, uint64_t idx, uint64
     // first; beyond capacity, the term keeps its smallest primes
     const bool pending = !(pos < fb.max_factors && atomicCAS(&slots[pos], 0ull, (unsigned long long)p) == 0ull);
     if (__builtin_expect(__any_sync(peers, pending), 0))
-        push_overflow(slots, fb.max_factors, p, pending, peers, leader);
+        push_overflow(slots, fb.max_factors, p, pending, peers);
 }
 
 // push out of line, for the baby-step families (doubling, fixed-n): one call
@@ -117,6 +121,16 @@ __device__ __forceinline__ void push(const FactorsView &fb, uint64_t idx, uint64
 // site, walks of a few blocks ran 24 % slower), while an out-of-line push in
 // the Smarandache walk's loop cost it 2.5x, so the others keep push inlined
 __device__ __noinline__ void push_call(const FactorsView &fb, uint64_t idx, uint64_t p) { push(fb, idx, p); }
+
+// Pushes p to the terms idx + j of the bits j of hits.  Lanes push their own
+// next term at the same time, so a warp takes as many pushes as its busiest
+// lane has: with a push wherever some lane has a zero, the primes below 137
+// took 80 pushes, one after another, for 80 terms.
+__device__ __noinline__ void push_bits(const FactorsView &fb, uint64_t idx, uint32_t hits, uint64_t p)
+{
+    for (; hits; hits &= hits - 1)
+        push(fb, idx + (uint32_t)(__ffs(hits) - 1), p);
+}
 
 // ------------------------------------------------------- step primitives
 // For p < 2^63 the modular double / add is: v = a + b - p (one 3-input add
@@ -547,7 +561,7 @@ __device__ __forceinline__ void run_doubling(const JobView &job, uint64_t p, uin
         const uint64_t k = job.param < p ? job.param : job.param % p;
         return m.mul(U, k);
     };
-    if (p < (1ull << 63) && (e - s) / BS >= 2 && job.variant != CTD_VARIANT_WALK) {
+    if (p < (1ull << 63) && e - s >= BS && job.variant != CTD_VARIANT_WALK) {
         // Walk w(n) = 2^-n instead: k 2^n = -1 (Proth) / 1 (Riesel, Mersenne
         // with k = 1) mod p iff w(n) = -k / k, a fixed target, and the giant
         // step w -> w 2^-32 is one reduction on the multiply pipe (redc32).
@@ -569,20 +583,20 @@ __device__ __forceinline__ void run_doubling(const JobView &job, uint64_t p, uin
         const uint32_t one = (uint32_t)(p & 1);
         const uint64_t at0 = s - job.n0;  // index of the first term
         auto giant = [&](uint64_t x) { return redc32(x, plo, phi, pinv32, one); };
-        auto replay = [&](uint64_t v, uint64_t b) {
+        auto zeros = [&](uint64_t v, uint64_t b, uint32_t terms) {
+            uint32_t hits = 0;
 #pragma unroll 1
-            for (int j = 0; j < BS; ++j) {
-                if (v == wt)
-                    push_call(job.fb, at0 + b * BS + j, p);
+            for (uint32_t j = 0; j < terms; ++j) {
+                hits |= (v == wt ? 1u : 0u) << j;
                 v = half63(v, p);
             }
+            if (hits)
+                push_bits(job.fb, at0 + b * BS, hits, p);
         };
+        auto replay = [&](uint64_t v, uint64_t b) { zeros(v, b, BS); };
         w = run_blocks(tlo, w, nb, giant, replay);
-        for (uint64_t n = s + nb * BS; n < e; ++n) {  // the short tail, term by term
-            if (w == wt)
-                push_call(job.fb, n - job.n0, p);
-            w = half63(w, p);
-        }
+        if ((e - s) % BS && match32((uint32_t)w, tlo))  // the tail: a block cut short
+            zeros(w, nb, (uint32_t)((e - s) % BS));
     } else if (p < (1ull << 63))
         walk_add63<true>(start(), 0, target, p, s - job.n0, steps, job.fb);
     else
@@ -2044,16 +2058,19 @@ __device__ __forceinline__ void run_item(const JobView &job, uint64_t p, uint64_
         run_peano(job, p, s, e);
 }
 
-// one (prime, tile) item: item k is tile k mod tiles of prime k / tiles
+// one (prime, tile) item: tile after tile, the primes in the list's order, so
+// that a warp's lanes walk the same terms of neighbouring primes (and push a
+// term that every prime divides together)
 template <uint32_t FAM>
-__device__ __forceinline__ void residue_item(const JobView &job, const uint64_t *__restrict__ primes, uint64_t k)
+__device__ __forceinline__ void residue_item(const JobView &job, const uint64_t *__restrict__ primes, uint64_t nprimes,
+                                             uint64_t k)
 {
     if (job.tiles == 1) {
         run_item<FAM>(job, primes[k], job.n0, job.n1);
         return;
     }
-    const uint64_t i = k / job.tiles;
-    const uint64_t t = k - i * job.tiles;
+    const uint64_t t = k / nprimes;
+    const uint64_t i = k - t * nprimes;
     const uint64_t s = job.n0 + t * job.tile_len;
     const uint64_t e = s + job.tile_len < job.n1 ? s + job.tile_len : job.n1;
     if (s < e)
@@ -2073,7 +2090,7 @@ residue_kernel(JobView job, const uint64_t *__restrict__ primes, uint64_t nprime
     if (!next) {
         const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
         for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < items; k += stride)
-            residue_item<FAM>(job, primes, k);
+            residue_item<FAM>(job, primes, nprimes, k);
         return;
     }
     const uint32_t lane = threadIdx.x & 31u;
@@ -2085,7 +2102,7 @@ residue_kernel(JobView job, const uint64_t *__restrict__ primes, uint64_t nprime
         if (base >= items)
             break;
         if (base + lane < items)
-            residue_item<FAM>(job, primes, base + lane);
+            residue_item<FAM>(job, primes, nprimes, base + lane);
     }
 }
 

@@ -293,3 +293,21 @@ def test_sieve_whole_and_quarter_windows(eng, lo):
     hi = lo + 2 * sms * (1 << 20) + 777
     mid = (lo + hi) // 2
     assert np.array_equal(eng.sieve(lo, hi), np.concatenate([eng.sieve(lo, mid), eng.sieve(mid, hi)]))
+
+
+@pytest.mark.parametrize("max_factors", [1, 3, 32, 45])
+@pytest.mark.parametrize("f0,f1", [(0, 1 << 12), (1 << 20, (1 << 20) + (1 << 17))])
+def test_overflow_keeps_the_smallest(eng, max_factors, f0, f1):
+    # every prime divides T(1) = 0: the slots end up with the smallest of them
+    got = run_gpu(eng, O.TRIBONACCI, 0, 1, 40, f0, f1, max_factors)
+    assert text(got) == O.trial_factor(O.TRIBONACCI, 0, 1, 40, f0, f1, max_factors, threads=1).format()
+
+
+@pytest.mark.parametrize("family,param", [(O.PROTH, 1279), (O.RIESEL, 7), (O.MERSENNE, 0), (O.SMARANDACHE, 10),
+                                          (O.FIBONACCI, 0), (O.TRIBONACCI, 0), (O.PROTH_FIXED_N, 7)])
+@pytest.mark.parametrize("terms", [79, 80, 81, 1023, 1024, 1500, 3000])
+def test_short_lists_in_tiles(eng, family, param, terms):
+    # fewer primes than threads: the index range is cut into short tiles
+    for f0, f1 in ((0, 300), ((1 << 33) + 1, (1 << 33) + 3000)):
+        got = run_gpu(eng, family, param, 3, 3 + terms, f0, f1)
+        assert text(got) == O.trial_factor(family, param, 3, 3 + terms, f0, f1, 32, threads=1).format()
