@@ -62,6 +62,24 @@ CTD_HD uint64_t dblmod(uint64_t a, uint64_t p)
     return a < p - a ? a << 1 : a - (p - a);
 }
 
+// 2^64 mod p.  On the device, for 2^31 <= p < 2^62, by two quotients in single
+// precision, each from below: inv is 1/p less at most 1.5 2^-20 of it (p
+// rounded up, the quotient within 2 ulp, then a factor 1 - 2^-20), so the first
+// leaves 2^64 - q p < 2^45 + p, the second less than 1.04 p.  (A 64-bit
+// remainder is a hundred instructions, and every kernel's set-up takes one.)
+CTD_HD uint64_t r_mod(uint64_t p)
+{
+#ifdef __CUDA_ARCH__
+    if ((p >> 31) && !(p >> 62)) {
+        const float inv = __fmul_rn(__fdividef(1.0f, __ull2float_ru(p)), 0.99999905f);
+        uint64_t r = (uint64_t)0 - __float2ull_rd(__fmul_rd(inv, 18446744073709551616.0f)) * p;
+        r -= __float2ull_rd(__fmul_rd(__ull2float_rd(r), inv)) * p;
+        return r >= p ? r - p : r;
+    }
+#endif
+    return ((uint64_t)0 - p) % p;
+}
+
 // ------------------------------------------------------- Montgomery, R=2^64
 // a b R^-1 mod p for a, b < p < 2^40, from 32-bit pieces: a = a1 2^32 + a0
 // with a1 < 2^9, so the product T = a b < 2^82 takes three multiply-adds
@@ -129,7 +147,7 @@ struct MontT {
     {
         p = modulus;
         pinv = neg_inverse(p);
-        one = ((uint64_t)0 - p) % p;  // 2^64 mod p
+        one = r_mod(p);
         r2 = 0;
     }
 

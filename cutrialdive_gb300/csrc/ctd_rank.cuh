@@ -28,6 +28,7 @@ constexpr uint32_t RANK_SPAN = 1u << 15;     // even numbers a tile's D's may sp
 constexpr uint32_t RANK_WORDS = RANK_SPAN / 16 + 2;  // two bits (p = D + 1, p = D - 1) an even number
 constexpr uint32_t RANK_BY_PRIME = 17;       // table primes below 64: divided prime by prime
 constexpr uint32_t RANK_BY_WARP = 171;       // table primes below 1024: a warp walks their multiples
+constexpr int RANK_CTAS = 5;                 // a SM: 42 KiB of shared memory, 48 registers a thread
 constexpr uint32_t RANK_HITS = 3 * RANK_TILE / 2;
 static_assert(RANK_TILE == 1u << 10 && TRIAL_PRIMES < 1u << 22, "a noted multiple is 32 bits");
 // Index ranges below e from which the tiles of ranks are taken instead of the
@@ -499,7 +500,7 @@ __device__ __forceinline__ void rank_tile_powers(const JobView &job, const RankL
 // 1.82 ms here with the multiples divided out where they are met, 0.92 with
 // them noted first, 0.74 + 0.13 with the last ranks in their own kernel.
 template <uint32_t FAM>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(256, RANK_CTAS)
 rank_kernel(JobView job, const uint64_t *__restrict__ primes, uint64_t nprimes, uint32_t tile, unsigned long long *next,
             RankList list)
 {
@@ -566,7 +567,7 @@ static cudaError_t launch_ranks(const JobView &v, const uint64_t *d_primes, uint
     if (e != cudaSuccess)
         return e;
     // a short list in small tiles, so that every CTA has one
-    const uint64_t grid = (uint64_t)sm_count * 4;
+    const uint64_t grid = (uint64_t)sm_count * RANK_CTAS;
     const uint64_t per = (n + grid - 1) / grid;
     const uint32_t tile = per < RANK_TILE ? (uint32_t)per : RANK_TILE;
     const uint64_t ntiles = (n + tile - 1) / tile;
