@@ -890,6 +890,7 @@ int ctd_run_plain(ctd_ctx *ctx, const ctd_job *job, uint32_t *counts_inout, uint
     if (rc)
         return rc;
     JobView view = make_view(job, ctx->d_counts, ctx->d_factors);
+    view.dense = 1;
     std::string err;
 
     uint64_t f0 = resume_after_prime ? resume_after_prime + 1 : job->f0;

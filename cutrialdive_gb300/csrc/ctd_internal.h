@@ -44,7 +44,7 @@ struct JobView {
     uint32_t variant;    // step form (CTD_VARIANT_*)
     uint32_t classify_min;  // doubling families: index ranges this long or longer walk power-residue classes
     uint32_t refine_q;   // largest rare prime whose character refines the classes (0: 61; < 11: none)
-    uint32_t pad;
+    uint32_t dense;      // the launch's list holds every prime of its range
     uint64_t param;      // k, n or base
     uint64_t n0, n1;     // index range of the factors buffer
     uint64_t tile_len;   // indices per tile (last tile may be shorter)
@@ -118,7 +118,7 @@ struct ClassCounters {
     uint32_t nrefine;               // primes listed for the rare-prime refinement (for their rank: Fibonacci, Lucas)
     uint32_t nlisted[8];            // primes the screen left for classification, by divisibility pattern
     uint32_t wide;                  // a prime of the launch is 2^40 or above
-    uint32_t nnine;                 // primes listed for the 9th-power character
+    uint32_t nnine;                 // primes listed for the 9th-power character (for their many hits: ranks)
 };
 // a prime with its class code (M << 16 | r)
 struct ClassItem {
@@ -137,7 +137,7 @@ struct ResidueScratch {
     uint32_t *nine = nullptr;    // indices of the primes for the 9th-power character
     uint64_t cap = 0;  // primes
     ClassCounters *counters = nullptr;
-    void *rank_items = nullptr;  // Fibonacci, Lucas: primes whose rank is left to take (RankItem)
+    void *rank_items = nullptr;  // Fibonacci, Lucas: primes whose rank is left to take (RankItem), then those with many hits (RankHits)
     uint32_t rank_cap = 0;
 };
 ResidueScratch *residue_scratch_create(int device, int sm_count);

@@ -19,6 +19,10 @@
 // W(2n) = W(n)^2 - 2 and W(2n+1) = W(n) W(n+1) + 3, and F(n) = 0 iff W(n) = 2
 // (t + 1/t = 2 only for t = 1): two products a bit of n, one a factor of 2,
 // where the doubling of (F(n), F(n+1)) takes three and more additions.
+//
+// Mersenne numbers go the same way: p | 2^n - 1 iff the order of 2 divides n,
+// and the order divides D = p - 1 (and a hit needs it below e); the power is
+// 2^-n, one product a bit (half_power).
 #pragma once
 
 namespace ctd {
@@ -37,7 +41,13 @@ static_assert(RANK_TILE == 1u << 10 && TRIAL_PRIMES < 1u << 22, "a noted multipl
 // they cost 2.14 (walk 2.14) and 2.17 (walk 2.40).  The primes below e cost a
 // tile about as much as 1/256 of e terms.
 constexpr uint64_t RANK_MIN_TERMS = 1024;
-__host__ __device__ constexpr uint64_t rank_min_terms(uint64_t e) { return RANK_MIN_TERMS + (e >> 8); }
+constexpr uint64_t rank_min_terms(uint64_t e) { return RANK_MIN_TERMS + (e >> 8); }
+// Mersenne, against the block walk: on the primes of a 2^28-wide range at 2^31,
+// 2000 terms from n = 1 take 1.53 ms (the walk 1.47) and 3000 take 1.59 (1.82);
+// from n = 40001, 3000 take 2.28 (2.03) and 5000 take 2.32 (2.73).  From 8192
+// terms on the walk over classes takes 5.7 ms, 13.0 for 100,000 terms, where the
+// orders take 1.7 and 3.0.
+constexpr uint64_t order_min_terms(uint64_t e) { return 2100 + e / 24; }
 
 // x mod q for x < 2^62, q < 2^20, with z = floor(2^32 / q): the high word,
 // then the low word in pieces that keep the running value below 2^32
@@ -52,6 +62,16 @@ __device__ __forceinline__ uint32_t rank_mod(uint64_t x, uint32_t q, uint32_t z)
     r = red(r << 12 | lo >> 20);
     r = red(r << 12 | (lo >> 8 & 0xfffu));
     return red(r << 8 | (lo & 0xffu));
+}
+
+// whether D = p + 1 (Fibonacci, Lucas: p = +-2 mod 5), else D = p - 1
+template <uint32_t FAM>
+__device__ __forceinline__ bool rank_above(uint64_t p)
+{
+    if (FAM == MERSENNE)
+        return false;
+    const uint32_t r5 = (uint32_t)(p % 5);
+    return r5 == 2 || r5 == 3;
 }
 
 // the sequence W modulo p, values in Montgomery form.  Below 2^40 the values
@@ -96,6 +116,21 @@ struct RankPowers {
     }
 };
 
+// 2^n - 1 modulo p
+template <bool NARROW>
+struct OrderPowers {
+    uint64_t p, pinv;
+
+    __device__ __forceinline__ void init(uint64_t modulus)
+    {
+        p = modulus;
+        pinv = Mont::neg_inverse(p);
+    }
+    __device__ __forceinline__ bool zero_at(uint64_t n) const { return half_power<NARROW>(p, pinv, n) == 1; }
+};
+template <uint32_t FAM, bool NARROW>
+using FamilyPowers = std::conditional_t<FAM == MERSENNE, OrderPowers<NARROW>, RankPowers<NARROW>>;
+
 // q^-1 mod 2^64 for odd q
 __device__ __forceinline__ uint64_t rank_inverse(uint32_t q)
 {
@@ -112,13 +147,13 @@ __device__ __forceinline__ uint64_t rank_without(uint64_t n, uint32_t q)
     return n;
 }
 
-// a(p), which divides S, or 0 when it exceeds amax; q1 > q2 the two largest
+// a(p) (Mersenne: the order of 2), which divides S, or 0 when it exceeds amax; q1 > q2 the two largest
 // odd primes of S (0: none).  A prime at a time is taken out of S while F
 // stays zero; what stays is final, and more than amax of it ends the search.
-template <bool NARROW>
+template <uint32_t FAM, bool NARROW>
 __device__ __noinline__ uint64_t rank_of(uint64_t p, uint64_t S, uint32_t q1, uint32_t q2, uint64_t amax)
 {
-    RankPowers<NARROW> w;
+    FamilyPowers<FAM, NARROW> w;
     w.init(p);
     uint64_t a = S, fixed = 1;
     auto reduce = [&](uint64_t q) {
@@ -154,53 +189,61 @@ __device__ __noinline__ uint64_t rank_of(uint64_t p, uint64_t S, uint32_t q1, ui
     return a <= amax ? a : 0;
 }
 
+// The primes whose rank is left to take, a few in a hundred, go to a list
+// that a second kernel works off: in the tile they kept one warp busy for
+// several powers while the CTA waited (0.92 ms for the tiles of a 2^26-wide
+// segment at 2^34).  Primes with many hits (small ones: 3 divides every second
+// 2^n - 1) go on to a third kernel, which spreads a prime's hits over the grid.
+struct RankItem {
+    uint64_t p, S;
+    unsigned long long top;
+};
+struct RankHits {
+    uint64_t p, first, a;  // n = first, first + a, ...
+};
+constexpr uint32_t RANK_MANY = 64;         // hits
+constexpr uint32_t RANK_HEAVY = 1u << 16;  // room for primes with as many; the others push their own
+struct RankList {
+    RankItem *items;
+    uint32_t *count;  // may exceed cap: the items beyond it were taken in their tiles
+    uint32_t cap;
+    RankHits *heavy;
+    uint32_t *nheavy;  // may exceed heavy_cap
+    uint32_t heavy_cap;
+};
+
 // The hits of the lanes' primes (those with mine; the whole warp calls):
 // n = a, 2a, ... or a/2, 3a/2, ...
 template <uint32_t FAM, bool NARROW>
-__device__ __noinline__ void rank_push(const JobView &job, bool mine, uint64_t p, uint64_t S, unsigned long long top)
+__device__ __noinline__ void rank_push(const JobView &job, const RankList &list, bool mine, uint64_t p, uint64_t S,
+                                       unsigned long long top)
 {
     const uint64_t s = job.n0, e = job.n1;
-    const uint64_t amax = FAM == FIBONACCI ? e - 1 : 2 * (e - 1);
+    const uint64_t amax = FAM == LUCAS ? 2 * (e - 1) : e - 1;
     uint64_t a = 0;
     if (mine)  // a(5) = 5; no Lucas number is a multiple of 5
-        a = p == 5 ? 5 : rank_of<NARROW>(p, S, (uint32_t)(top >> 32), (uint32_t)top, amax);
+        a = FAM != MERSENNE && p == 5 ? 5 : rank_of<FAM, NARROW>(p, S, (uint32_t)(top >> 32), (uint32_t)top, amax);
     if (a > amax || (FAM == LUCAS && (a & 1)))
         a = 0;
     // first hit n = h mod a, and how many
     uint64_t first = 0, hits = 0;
     if (a) {
-        const uint64_t h = FAM == FIBONACCI ? 0 : a >> 1, r = s % a;
+        const uint64_t h = FAM == LUCAS ? a >> 1 : 0, r = s % a;
         first = s + (h >= r ? h - r : a - r + h);
         hits = first < e ? (e - 1 - first) / a + 1 : 0;
     }
-    // few hits: every lane pushes its own; many: the warp a lane's together
-    const uint32_t lane = threadIdx.x & 31u;
-    if (hits <= 8)
-        for (uint64_t i = 0; i < hits; ++i)
-            push(job.fb, first + i * a - s, p);
-    __syncwarp();
-    for (uint32_t todo = __ballot_sync(0xffffffffu, hits > 8); todo; todo &= todo - 1) {
-        const int from = __ffs(todo) - 1;
-        const uint64_t pk = __shfl_sync(0xffffffffu, p, from), ak = __shfl_sync(0xffffffffu, a, from);
-        for (uint64_t x = __shfl_sync(0xffffffffu, first, from) + lane * ak; x < e; x += 32 * ak)
-            push(job.fb, x - s, pk);
-        __syncwarp();
+    if (hits > RANK_MANY) {
+        const uint32_t at = atomicAdd(list.nheavy, 1u);
+        if (at < list.heavy_cap) {
+            list.heavy[at] = RankHits{p, first, a};
+            hits = 0;
+        }
     }
+    // every lane pushes its own
+    for (uint64_t i = 0; i < hits; ++i)
+        push(job.fb, first + i * a - s, p);
+    __syncwarp();
 }
-
-// The primes whose rank is left to take, a few in a hundred, go to a list
-// that a second kernel works off: in the tile they kept one warp busy for
-// several powers while the CTA waited (0.92 ms for the tiles of a 2^26-wide
-// segment at 2^34).
-struct RankItem {
-    uint64_t p, S;
-    unsigned long long top;
-};
-struct RankList {
-    RankItem *items;
-    uint32_t *count;  // may exceed cap: the items beyond it were taken in their tiles
-    uint32_t cap;
-};
 
 struct RankShared {
     uint64_t p[RANK_TILE];
@@ -277,8 +320,7 @@ __device__ bool rank_tile(const JobView &job, const RankList &list, RankShared &
     // mark the D's: bit 2i for p = D + 1, bit 2i + 1 for p = D - 1
     for (uint32_t i = tid; i < n; i += 256) {
         const uint64_t p = primes[i];
-        const uint32_t r5 = (uint32_t)(p % 5);
-        const bool up = r5 == 2 || r5 == 3;
+        const bool up = rank_above<FAM>(p);
         const uint32_t pos = 2 * (uint32_t)(((up ? p + 1 : p - 1) - m0) >> 1) + up;
         if (atomicOr(&sh.bits[pos >> 5], 1u << (pos & 31)) >> (pos & 31) & 1)
             sh.flags = 1;
@@ -314,8 +356,7 @@ __device__ bool rank_tile(const JobView &job, const RankList &list, RankShared &
     // smallest primes of their D's
     for (uint32_t i = tid; i < n; i += 256) {
         const uint64_t p = primes[i];
-        const uint32_t r5 = (uint32_t)(p % 5);
-        const bool up = r5 == 2 || r5 == 3;
+        const bool up = rank_above<FAM>(p);
         const uint64_t D = up ? p + 1 : p - 1;
         const uint32_t pos = 2 * (uint32_t)((D - m0) >> 1) + up;
         const uint32_t slot = sh.before[pos >> 5] + __popc(sh.bits[pos >> 5] & ((1u << (pos & 31)) - 1u));
@@ -345,9 +386,8 @@ __device__ bool rank_tile(const JobView &job, const RankList &list, RankShared &
     auto divide_out = [&](uint32_t slot, uint32_t k) {
         const uint4 t = g_trial_div[k];
         const uint64_t inv = (uint64_t)t.y << 32 | t.x, p = sh.p[slot];
-        const uint32_t r5 = (uint32_t)(p % 5);
         unsigned long long power = t.w;
-        for (uint64_t x = (r5 == 2 || r5 == 3 ? p + 1 : p - 1) * inv * inv; __umul64hi(x, t.w) == 0; x *= inv)
+        for (uint64_t x = (rank_above<FAM>(p) ? p + 1 : p - 1) * inv * inv; __umul64hi(x, t.w) == 0; x *= inv)
             power *= t.w;
         unsigned long long *const S = (unsigned long long *)&sh.S[slot], *const top = &sh.top[slot];
         for (unsigned long long old = *S, was; (was = atomicCAS(S, old, old * power)) != old; old = was) {
@@ -413,7 +453,7 @@ template <uint32_t FAM, bool NARROW>
 __device__ __forceinline__ void rank_tile_powers(const JobView &job, const RankList &list, RankShared &sh, uint32_t n)
 {
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint64_t amax = FAM == FIBONACCI ? job.n1 - 1 : 2 * (job.n1 - 1);
+    const uint64_t amax = FAM == LUCAS ? 2 * (job.n1 - 1) : job.n1 - 1;
     constexpr uint32_t SLOT = 0x7ffu, SMOOTH = 0x800u;
     // exponents, and their lengths counted
     for (uint32_t i = tid; i < n; i += 256) {
@@ -421,7 +461,7 @@ __device__ __forceinline__ void rank_tile_powers(const JobView &job, const RankL
         const uint32_t q1 = (uint32_t)(sh.top[i] >> 32), q2 = (uint32_t)sh.top[i];
         const bool smooth = S >= p - 1;
         uint64_t E = S;
-        if (p == 5) {
+        if (FAM != MERSENNE && p == 5) {
             E = 0;
             sh.finish[atomicAdd(&sh.nfinish, 1u)] = (uint16_t)i;
         } else if (smooth) {
@@ -460,7 +500,7 @@ __device__ __forceinline__ void rank_tile_powers(const JobView &job, const RankL
     __syncthreads();
     for (uint32_t k = tid; k < npow; k += 256) {
         const uint32_t o = sh.order[k], i = o & SLOT;
-        RankPowers<NARROW> w;
+        FamilyPowers<FAM, NARROW> w;
         w.init(sh.p[i]);
         if (w.zero_at(sh.E[i]))
             sh.finish[atomicAdd(&sh.nfinish, 1u)] = (uint16_t)i;
@@ -471,7 +511,7 @@ __device__ __forceinline__ void rank_tile_powers(const JobView &job, const RankL
     const uint32_t nsecond = sh.nsecond;
     for (uint32_t k = tid; k < nsecond; k += 256) {
         const uint32_t i = sh.second[k];
-        RankPowers<NARROW> w;
+        FamilyPowers<FAM, NARROW> w;
         w.init(sh.p[i]);
         if (w.zero_at(rank_without(sh.S[i], (uint32_t)sh.top[i])))
             sh.finish[atomicAdd(&sh.nfinish, 1u)] = (uint16_t)i;
@@ -488,7 +528,33 @@ __device__ __forceinline__ void rank_tile_powers(const JobView &job, const RankL
         if (k < nfinish && !mine)
             list.items[at] = RankItem{sh.p[i], sh.S[i], sh.top[i]};
         if (__any_sync(0xffffffffu, mine))
-            rank_push<FAM, NARROW>(job, mine, sh.p[i], sh.S[i], sh.top[i]);
+            rank_push<FAM, NARROW>(job, list, mine, sh.p[i], sh.S[i], sh.top[i]);
+    }
+}
+
+// Mersenne: a tile's primes each by itself, p - 1 divided by every prime below e
+__device__ __noinline__ void rank_alone(const JobView &job, const RankList &list, const uint64_t *__restrict__ primes,
+                                        uint32_t n, uint32_t nq)
+{
+    for (uint32_t k = threadIdx.x; k < ((n + 31) & ~31u); k += 256) {
+        const uint64_t p = k < n ? primes[k] : 3, D = p - 1;
+        uint64_t S = D & (0 - D);
+        unsigned long long top = 0;
+        for (uint32_t i = 0; i < nq; ++i) {
+            const uint4 t = g_trial_div[i];
+            const uint64_t inv = (uint64_t)t.y << 32 | t.x;
+            uint64_t x = D * inv;
+            if (__umul64hi(x, t.w) != 0)
+                continue;
+            do {
+                S *= t.w;
+                x *= inv;
+            } while (__umul64hi(x, t.w) == 0);
+            top = (unsigned long long)t.w << 32 | top >> 32;
+        }
+        OrderPowers<false> w;
+        w.init(p);
+        rank_push<MERSENNE, false>(job, list, k < n && w.zero_at(S), p, S, top);
     }
 }
 
@@ -520,8 +586,11 @@ rank_kernel(JobView job, const uint64_t *__restrict__ primes, uint64_t nprimes, 
         const uint32_t n = (uint32_t)(nprimes - first < tile ? nprimes - first : tile);
         if (!rank_tile<FAM>(job, list, sh, primes + first, n, nq)) {
             // a sparse or unordered stretch of the list: item by item
-            for (uint64_t k = threadIdx.x; k < (uint64_t)n * job.tiles; k += 256)
-                residue_item<FAM>(job, primes + first, n, k);
+            if constexpr (FAM == MERSENNE)  // (its walks' filter has no room here)
+                rank_alone(job, list, primes + first, n, nq);
+            else
+                for (uint64_t k = threadIdx.x; k < (uint64_t)n * job.tiles; k += 256)
+                    residue_item<FAM>(job, primes + first, n, k);
         }
     }
 }
@@ -535,17 +604,30 @@ __global__ void __launch_bounds__(256) rank_finish_kernel(JobView job, RankList 
         const bool mine = k < n;
         const RankItem it = mine ? list.items[k] : RankItem{0, 0, 0};
         if (__any_sync(0xffffffffu, it.p >= MONT_NARROW_LIMIT))
-            rank_push<FAM, false>(job, mine, it.p, it.S, it.top);
+            rank_push<FAM, false>(job, list, mine, it.p, it.S, it.top);
         else
-            rank_push<FAM, true>(job, mine, it.p, it.S, it.top);
+            rank_push<FAM, true>(job, list, mine, it.p, it.S, it.top);
+    }
+}
+
+// the hits of the primes that have many, 32 chunks of each prime's over the warps
+__global__ void __launch_bounds__(256) rank_heavy_kernel(JobView job, RankList list)
+{
+    constexpr uint32_t CHUNKS = 32;
+    const uint32_t n = *list.nheavy < list.heavy_cap ? *list.nheavy : list.heavy_cap, lane = threadIdx.x & 31u;
+    for (uint32_t id = (blockIdx.x * 256 + threadIdx.x) >> 5; id < n * CHUNKS; id += gridDim.x * 8) {
+        const RankHits h = list.heavy[id % n];
+        for (uint64_t x = h.first + (id / n * 32 + lane) * h.a; x < job.n1; x += CHUNKS * 32 * h.a)
+            push(job.fb, x - job.n0, h.p);
     }
 }
 
 // whether a job's primes go by tiles of ranks
 inline bool takes_ranks(const JobView &v)
 {
-    return (v.family == FIBONACCI || v.family == LUCAS) && v.variant == CTD_VARIANT_AUTO && v.n0 >= 1 &&
-           v.n1 <= TRIAL_LIMIT && v.n1 - v.n0 >= rank_min_terms(v.n1);
+    const bool mersenne = v.family == MERSENNE && v.dense;
+    return (v.family == FIBONACCI || v.family == LUCAS || mersenne) && v.variant == CTD_VARIANT_AUTO && v.n0 >= 1 &&
+           v.n1 <= TRIAL_LIMIT && v.n1 - v.n0 >= (mersenne ? order_min_terms(v.n1) : rank_min_terms(v.n1));
 }
 
 // room for the list: a few in a hundred primes are listed at 2^34, half of
@@ -579,6 +661,11 @@ static cudaError_t launch_ranks(const JobView &v, const uint64_t *d_primes, uint
     note_kernel_launch();
     const uint64_t blocks = ((list.cap < n ? list.cap : n) + 255) / 256;
     rank_finish_kernel<FAM><<<(unsigned)(blocks < grid ? blocks : grid), 256, 0, st>>>(v, list);
+    e = cudaGetLastError();
+    if (e != cudaSuccess)
+        return e;
+    note_kernel_launch();
+    rank_heavy_kernel<<<(unsigned)sm_count * 4, 256, 0, st>>>(v, list);
     return cudaGetLastError();
 }
 

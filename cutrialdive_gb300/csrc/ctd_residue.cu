@@ -22,6 +22,7 @@
 #include <atomic>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 namespace ctd {
@@ -3257,6 +3258,38 @@ int launch_residues(const JobView &view, const uint64_t *d_primes, uint64_t npri
 {
     if (!nprimes || view.n1 <= view.n0)
         return CTD_OK;
+    if (scratch && takes_ranks(view)) {
+        const int rc0 = ensure_class_scratch(scratch, 0, err);  // its counters
+        if (rc0)
+            return rc0;
+        const uint32_t cap = rank_list_cap(nprimes);
+        if (cap > scratch->rank_cap) {
+            cudaFree(scratch->rank_items);
+            scratch->rank_items = nullptr;
+            scratch->rank_cap = 0;
+            if (cudaMalloc(&scratch->rank_items, cap * sizeof(RankItem) + RANK_HEAVY * sizeof(RankHits)) == cudaSuccess)
+                scratch->rank_cap = cap;
+            else  // the tiles finish their primes themselves
+                (void)cudaGetLastError();
+        }
+        RankItem *const items = (RankItem *)scratch->rank_items;
+        const RankList list{items, &scratch->counters->nrefine, scratch->rank_cap,
+                            (RankHits *)(items + scratch->rank_cap), &scratch->counters->nnine,
+                            scratch->rank_cap ? RANK_HEAVY : 0u};
+        cudaError_t rc;
+        if (view.family == FIBONACCI)
+            rc = launch_ranks<FIBONACCI>(view, d_primes, nprimes, scratch->sm_count, stream, scratch->counters, list);
+        else if (view.family == LUCAS)
+            rc = launch_ranks<LUCAS>(view, d_primes, nprimes, scratch->sm_count, stream, scratch->counters, list);
+        else
+            rc = launch_ranks<MERSENNE>(view, d_primes, nprimes, scratch->sm_count, stream, scratch->counters, list);
+        if (rc != cudaSuccess) {
+            err = std::string("rank kernel launch: ") + cudaGetErrorString(rc);
+            return CTD_ERR_CUDA;
+        }
+        note_kernel_launch();
+        return CTD_OK;
+    }
     const bool doubling = view.family == PROTH || view.family == RIESEL || view.family == MERSENNE;
     const uint32_t cmin = view.classify_min ? view.classify_min : DEFAULT_CLASSIFY_MIN;
     // (the class passes index the primes with 32 bits)
@@ -3288,28 +3321,6 @@ int launch_residues(const JobView &view, const uint64_t *d_primes, uint64_t npri
         next = &scratch->counters->next;
     }
     cudaError_t rc;
-    if (next && takes_ranks(view)) {
-        const uint32_t cap = rank_list_cap(nprimes);
-        if (cap > scratch->rank_cap) {
-            cudaFree(scratch->rank_items);
-            scratch->rank_items = nullptr;
-            scratch->rank_cap = 0;
-            if (cudaMalloc(&scratch->rank_items, (size_t)cap * sizeof(RankItem)) == cudaSuccess)
-                scratch->rank_cap = cap;
-            else  // the tiles finish their primes themselves
-                (void)cudaGetLastError();
-        }
-        const RankList list{(RankItem *)scratch->rank_items, &scratch->counters->nrefine, scratch->rank_cap};
-        rc = view.family == FIBONACCI
-                 ? launch_ranks<FIBONACCI>(view, d_primes, nprimes, scratch->sm_count, stream, scratch->counters, list)
-                 : launch_ranks<LUCAS>(view, d_primes, nprimes, scratch->sm_count, stream, scratch->counters, list);
-        if (rc != cudaSuccess) {
-            err = std::string("rank kernel launch: ") + cudaGetErrorString(rc);
-            return CTD_ERR_CUDA;
-        }
-        note_kernel_launch();
-        return CTD_OK;
-    }
     switch (view.family) {
     case MERSENNE: rc = launch_fam<MERSENNE>(view, d_primes, nprimes, grid, block, stream, next); break;
     case PROTH: rc = launch_fam<PROTH>(view, d_primes, nprimes, grid, block, stream, next); break;

@@ -122,7 +122,8 @@ typedef struct ctd_tuning {
 
 /* Step forms a tuning can select.  AUTO: the fastest measured form for the
  * family and prime width.  WALK: the term-by-term walk (doubling families:
- * no baby-step blocks and no power-residue classes; fixed-n families: the
+ * no baby-step blocks, no power-residue classes and, Mersenne, no orders of
+ * 2; fixed-n families: the
  * walk instead of the closed-form solve; Fibonacci/Lucas: no rank of
  * apparition; tribonacci: one term after the other instead of blocks around
  * a centre; Smarandache: the 64-bit Shoup step instead of the 32-bit Barrett
