@@ -1671,14 +1671,13 @@ __device__ __forceinline__ uint64_t smarandache_walk_b32(const JobView &job, uin
 // a term's test is one multiply-add of x by p^-1 M^i, the running word
 // C_i(m) p^-1 added, and one compare, and only every J-th state is computed:
 // x(m+J) = W x + D(m), W = M^J mod p by Shoup's quotient (two of its products
-// are single-width), D(m) = C_J(m) mod p by a modular addition.  SM_GROUP
-// blocks share a vote; a group with a candidate is stepped exactly.
+// are single-width), D(m) = C_J(m) mod p by a modular addition.  A
+// group of blocks shares a vote; a group with a candidate is stepped exactly.
 //
 // Bound by integer issue (5.8 instructions a term for J = 3, 7.1 for J = 2) and
 // the multiply pipe: 4 + J slots a block (the high product takes two) where a
 // step a term took 4 a term.  Base 10, n = 10..999, the primes of a 2^26-wide
 // segment below 2^28: 1.48 ms with a step a term, 1.13 here.
-constexpr int SM_GROUP = 4;
 
 // Exact steps m -> m + 1, `count` of them, from x = S(m) < 3p: the terms
 // m .. m + count - 1 pushed where they are zeros.  Returns the last state.
@@ -1703,7 +1702,8 @@ __device__ __noinline__ uint32_t smarandache_blocks32(const JobView &job, Mont32
     const uint32_t p = (uint32_t)mt.p, pinv = 0u - (uint32_t)mt.pinv;
     const uint64_t Mf = mt.to(M);
     const uint32_t Ms = mt.shoup_of_form(Mf);
-    const uint32_t groups = steps / (SM_GROUP * J);
+    constexpr int GROUP = J == 1 ? 16 : 8;
+    const uint32_t groups = steps / (GROUP * J);
     if (groups) {
         // c[i] = C_i(m) p^-1, from C_0 = 0, C_{i+1}(m) = M C_i(m) + m + i + 1;
         // per block C_i grows by J (M^i - 1) / (M - 1)
@@ -1738,7 +1738,7 @@ __device__ __noinline__ uint32_t smarandache_blocks32(const JobView &job, Mont32
                 x0 = x;
                 bool cand = false;
 #pragma unroll
-                for (int b = 0; b < SM_GROUP; ++b) {
+                for (int b = 0; b < GROUP; ++b) {
 #pragma unroll
                     for (int i = 0; i < J; ++i) {
                         cand |= (i ? x * mul[i] + c[i] : x * pinv) < thr[i];
@@ -1753,10 +1753,10 @@ __device__ __noinline__ uint32_t smarandache_blocks32(const JobView &job, Mont32
                 hit = __any_sync(__activemask(), cand);
             } while (++g < groups && !hit);
             if (hit)
-                smarandache_exact32(job.fb, job.n0, p, x0, M, Ms, m + (g - 1) * (SM_GROUP * J), SM_GROUP * J);
+                smarandache_exact32(job.fb, job.n0, p, x0, M, Ms, m + (g - 1) * (GROUP * J), GROUP * J);
         }
-        m += groups * (SM_GROUP * J);
-        steps -= groups * (SM_GROUP * J);
+        m += groups * (GROUP * J);
+        steps -= groups * (GROUP * J);
     }
     return smarandache_exact32(job.fb, job.n0, p, x, M, Ms, m, steps);
 }
@@ -1778,8 +1778,8 @@ __device__ __noinline__ uint32_t smarandache_blocks32(const JobView &job, Mont32
 // A walk of S itself adds m in the wide product and compares with 0, p, 2p.
 // Bound by the multiply pipe (a wide product with a 64-bit sum takes nearly
 // three slots).  The primes of a 2^25-wide range at 2^34: base 10, n = 2001 ..
-// 8999 (J = 2), 4.40 ms, 6.8 with the walk of S; base 7, n = 20001 .. 24321
-// (J = 1), 3.99 and 4.50.
+// 8999 (J = 2), 4.32 ms, 6.8 with the walk of S; base 7, n = 20001 .. 24321
+// (J = 1), 3.89 and 4.50.
 __device__ __noinline__ uint64_t smarandache_exact64(FactorsView fb, uint64_t n0, uint64_t p, uint64_t Y, uint64_t t,
                                                      uint64_t dt, uint32_t M, uint64_t Ms, uint64_t m, uint32_t count)
 {
@@ -1807,7 +1807,7 @@ __device__ __noinline__ uint64_t smarandache_blocks64(const JobView &job, uint64
                                                          uint64_t t, uint64_t dt, uint32_t M, uint64_t Ms, uint64_t Ws,
                                                          uint64_t m, uint32_t steps)
 {
-    constexpr int GROUP = J == 1 ? 8 : SM_GROUP;
+    constexpr int GROUP = J == 1 ? 16 : J == 2 ? 8 : 4;
     const uint32_t groups = steps / (GROUP * J);
     if (groups) {
         const int sh = 63 - clz64(p);
