@@ -89,36 +89,37 @@ FAMILY_NAMES = {0: "MERSENNE", 1: "PROTH", 2: "RIESEL", 3: "SMARANDACHE", 4: "FI
 #    [2^32, 2^32 + 2^27) of this workload
 #    (6,047,768 primes; the capture's command is in the profile summary);
 #    the live launch time comes from CUDA events in this run.
-#  * smarandache -- the 32-bit Shoup step (p < 2^30): three 32-bit
-#    multiplies per update (the quotient's high half, x M and q p), against
-#    the integer multiply-add rate measured now;
-#  * linear -- the dominant tribonacci launch: lazily reduced blocks of 18
-#    steps, a three-input 64-bit add (2) and the compare (1) per step plus 3
-#    shifts per block = 57/18 ALU operations per update, against the ALU
-#    compare rate measured now.
+#  * smarandache -- blocks of 32-bit Shoup steps (p < 2^30): a block of three
+#    terms (n < 100) takes three multiplies for its step and three for its
+#    tests, one of two terms (n >= 100) three and two: 2.45 per update over
+#    n = 10 .. 999, against the integer multiply-add rate measured now;
+#  * linear -- the dominant tribonacci launch: blocks of 31 terms, 28
+#    three-input sums, 25 half minima and maxima and 2 compares on the ALU =
+#    55/31 ALU operations per update, against the ALU compare rate measured
+#    now (the multiply pipe, with the blocks' jumps, is as busy).
 PROTH_NCU = {"primes": 6047768,
              # warp instructions x active lanes per instruction, one entry per launch
              "thread_inst": {
                  "screen_kernel": 65171117 * 29.81,
-                 "classify_kernel_p0": 132079999 * 29.59,
-                 "classify_kernel_p1": 296012527 * 28.57,
-                 "classify_kernel_p2": 50881891 * 29.24,
-                 "classify_kernel_p3": 113313117 * 27.48,
-                 "classify_kernel_p4": 32032031 * 29.39,
-                 "classify_kernel_p5": 70274163 * 27.39,
-                 "classify_kernel_p6": 12315032 * 28.47,
-                 "classify_kernel_p7": 27235315 * 26.17,
-                 "refine_kernel": 289309073 * 26.81,
-                 "nine_kernel": 85534542 * 28.53,
+                 "classify_kernel_p0": 109554151 * 29.03,
+                 "classify_kernel_p1": 241305487 * 28.09,
+                 "classify_kernel_p2": 40675533 * 28.53,
+                 "classify_kernel_p3": 93172111 * 26.93,
+                 "classify_kernel_p4": 26558798 * 28.83,
+                 "classify_kernel_p5": 58077851 * 26.84,
+                 "classify_kernel_p6": 10047747 * 27.71,
+                 "classify_kernel_p7": 22809306 * 25.60,
+                 "refine_kernel": 245981681 * 26.61,
+                 "nine_kernel": 79744251 * 28.19,
                  "regroup_kernel": 56933014 * 15.98,
-                 "class_walk_kernel": 1766393743 * 29.29},
+                 "class_walk_kernel": 1368855968 * 26.09},
              # dram__bytes_read.sum + dram__bytes_write.sum of the same launches, MB
-             "dram_bytes": (62.006784 + 14.746624 + 55.477248 + 5.529600 + 64.505856 + 8.557056 + 31.603712 +
-                            1.104896 + 47.789312 + 3.366144 + 21.782528 + 0.321280 + 36.367616 + 1.626624 + 8.100096
-                            + 0.015616 + 15.639552 + 0.112640 + 83.481600 + 1.313792 + 68.398080 + 0.144128 +
-                            73.165568 + 8.725248 + 53.848832 + 5.083648) * 1e6}
-SMARANDACHE_MULS_PER_UPDATE = 3
-TRIBONACCI_ALU_OPS_PER_UPDATE = 57 / 18
+             "dram_bytes": (62.127360 + 14.758912 + 55.779840 + 6.085888 + 64.821248 + 9.626880 + 31.815168 +
+                            1.307904 + 48.090112 + 3.739904 + 21.870336 + 0.407552 + 36.465152 + 1.719296 + 8.113152
+                            + 0.021248 + 15.670784 + 0.138752 + 83.027712 + 3.585792 + 68.413952 + 1.600256 +
+                            73.113856 + 11.770880 + 53.818624 + 3.506944) * 1e6}
+SMARANDACHE_MULS_PER_UPDATE = (90 * 2 + 900 * 2.5) / 990
+TRIBONACCI_ALU_OPS_PER_UPDATE = 55 / 31
 
 
 def mv_bound(y: int) -> int:
@@ -482,7 +483,7 @@ def run_ours(args, world, rank, local):
     elif wl.name == "smarandache":
         achieved = per_launch_updates * SMARANDACHE_MULS_PER_UPDATE / launch_s
         roofline = {
-            "bound": "int_multiply", "kernel": "residue_kernel<SMARANDACHE> (32-bit Shoup step)",
+            "bound": "int_multiply", "kernel": "residue_kernel<SMARANDACHE> (blocks of 32-bit Shoup steps)",
             "achieved": achieved / 1e9, "peak": (peaks["imad"] / 1e9) if peaks["imad"] else None,
             "unit": "Gmul/s", "frac": (achieved / peaks["imad"]) if peaks["imad"] else None,
             "muls_per_update": SMARANDACHE_MULS_PER_UPDATE, "launch_ms": launch_s * 1e3,
