@@ -391,6 +391,27 @@ struct TargetFilter {
         sl.x |= 1u << (t & 31);
         sl.y |= 1u << ((h >> 22) & 31);
     }
+    // The same with two bits in each word, for 64 targets in the 32 slots: a
+    // state that meets none passes with probability about 16 E[X^4] / 32^4 =
+    // 0.14 % for the X ~ Poisson(2) targets of its slot; with one bit in each
+    // word it is E[X^2] / 32^2 = 0.6 %.  3 2^n + 1, 100001 terms, the primes of
+    // 2^29 from 2^33: 12.85 ms with one bit in each word, 11.63 with a third
+    // bit, 11.28 with all four.  For 32 targets (0.2 % with two bits) four are
+    // no faster.
+    __device__ __forceinline__ void insert2(uint32_t t) const
+    {
+        const uint32_t h = t * FILTER_A;
+        uint2 &sl = slot(h);
+        sl.x |= 1u << (t & 31) | 1u << ((h >> 17) & 31);
+        sl.y |= 1u << ((h >> 22) & 31) | 1u << ((h >> 12) & 31);
+    }
+    __device__ __forceinline__ uint32_t test2(uint32_t lo) const
+    {
+        const uint32_t h = lo * FILTER_A;
+        const uint2 sl = slot(h);
+        return __funnelshift_r(sl.x, sl.x, lo) & __funnelshift_r(sl.x, sl.x, h >> 17) &
+               __funnelshift_r(sl.y, sl.y, h >> 22) & __funnelshift_r(sl.y, sl.y, h >> 12);
+    }
     // marks the 32 targets' low words
     __device__ __forceinline__ void build(const uint32_t (&tlo)[BS]) const
     {
@@ -705,23 +726,24 @@ __device__ __forceinline__ uint64_t half_form(const Mont &m, uint32_t M)
 // them all.  ng groups share a vote each; replay(z, b) settles block b of state
 // z.  Terms past the range's end are left to replay.
 //
-// Twice the targets in the same filter pass 3 times the states (0.6 %), so a
-// warp's block takes the exact compares every sixth time instead of every
-// sixteenth, but there are half the giant steps, tests and votes: worth the 32
-// more targets (some 900 instructions) from CLASS_LONG terms.
+// Blocks of 64 take half the giant steps, tests and votes, for 32 more targets
+// (some 1000 instructions): worth it from CLASS_LONG terms (1536 and 3500 are
+// within 0.4 % of it).  With the filter's four bits a vote of 2 blocks takes
+// the exact compares once in 11; 4 blocks a vote are 2 % slower.
 constexpr uint64_t CLASS_LONG = 2560;
+constexpr int CLASS_GROUP = 2;  // blocks of 64 a vote
 template <int B, class Giant, class Near, class Replay>
 __device__ __forceinline__ void class_blocks(const TargetFilter &flt, const uint32_t (&tlo)[BS], uint64_t x, uint32_t ng,
                                              Giant giant, Near near, Replay replay)
 {
-    constexpr int G = B == 64 ? 2 : FILTER_GROUP;
+    constexpr int G = B == 64 ? CLASS_GROUP : FILTER_GROUP;
     for (uint32_t g = 0; g < ng; ++g) {
         const uint64_t x0 = x;
         uint32_t fs[G], any = 0;
 #pragma unroll
         for (int i = 0; i < G; ++i) {
             x = giant(x);
-            fs[i] = flt.test((uint32_t)x) & 1;
+            fs[i] = (B == 64 ? flt.test2((uint32_t)x) : flt.test((uint32_t)x)) & 1;
             any |= fs[i];
         }
         if (__any_sync(__activemask(), any)) {
@@ -802,12 +824,12 @@ __device__ void run_doubling_class(const JobView &job, uint64_t p, uint32_t M, u
 #pragma unroll
         for (int j = 0; j < BS; ++j) {
             t = step.mul(t, p);
-            flt.insert((uint32_t)t);
+            flt.insert2((uint32_t)t);
             t = step.mul(t, p);
-            flt.insert((uint32_t)t);
+            flt.insert2((uint32_t)t);
             tlo[j] = (uint32_t)t;
         }
-        const uint32_t ng = (uint32_t)((cnt + 127) / 128);
+        const uint32_t ng = (uint32_t)((cnt + 64 * CLASS_GROUP - 1) / (64 * CLASS_GROUP));
         auto long_replay = [&](uint64_t z, uint64_t b) { replay(z, b * 64, 64); };
         if (M == 1) {
             class_blocks<64>(flt, tlo, w, ng, [&](uint64_t x) { return redc(redc(x)); }, near, long_replay);
