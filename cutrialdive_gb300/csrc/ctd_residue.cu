@@ -561,6 +561,20 @@ __device__ __forceinline__ uint64_t redc32(uint64_t u, uint32_t plo, uint32_t ph
     return (uint64_t)m * phi + h;
 }
 
+// u * 2^-M mod p for u < p, odd p < 2^63, 0 < M < 32: the same with the low M
+// bits, m = u_lo (-p^-1) mod 2^M, r = (u + m p) / 2^M < p.  Half the instructions
+// of a Shoup product: the class walk's targets by it take 3 2^n + 1, 100001
+// terms, the primes of 2^29 from 2^33, from 11.28 to 11.02 ms (50000 terms over
+// 2^30: 18.98 to 18.36).
+__device__ __forceinline__ uint64_t redc_bits(uint64_t u, uint32_t plo, uint32_t phi, uint32_t pinv32, uint32_t M)
+{
+    const uint32_t m = (uint32_t)u * pinv32 & ((1u << M) - 1);
+    const uint64_t s = (uint64_t)m * plo + u;  // below 2^63 + 2^63
+    const uint64_t h = (uint64_t)m * phi + (s >> 32);
+    return (uint64_t)__funnelshift_r((uint32_t)h, (uint32_t)(h >> 32), M) << 32 |
+           __funnelshift_r((uint32_t)s, (uint32_t)h, M);
+}
+
 // ------------------------------------------------------------- families
 
 // Proth k*2^n+1, Riesel k*2^n-1, Mersenne 2^n-1 (riesel_proth.hpp:90-115,
@@ -821,14 +835,20 @@ __device__ void run_doubling_class(const JobView &job, uint64_t p, uint32_t M, u
     // (the warp's lanes walk classes of about the same M: one block length)
     if (__any_sync(__activemask(), cnt >= CLASS_LONG)) {
         flt.clear();
+        auto mark = [&](auto next) {
 #pragma unroll
-        for (int j = 0; j < BS; ++j) {
-            t = step.mul(t, p);
-            flt.insert2((uint32_t)t);
-            t = step.mul(t, p);
-            flt.insert2((uint32_t)t);
-            tlo[j] = (uint32_t)t;
-        }
+            for (int j = 0; j < BS; ++j) {
+                t = next(t);
+                flt.insert2((uint32_t)t);
+                t = next(t);
+                flt.insert2((uint32_t)t);
+                tlo[j] = (uint32_t)t;
+            }
+        };
+        if (M < 32)
+            mark([&](uint64_t x) { return redc_bits(x, plo, phi, pinv32, M); });
+        else
+            mark([&](uint64_t x) { return step.mul(x, p); });
         const uint32_t ng = (uint32_t)((cnt + 64 * CLASS_GROUP - 1) / (64 * CLASS_GROUP));
         auto long_replay = [&](uint64_t z, uint64_t b) { replay(z, b * 64, 64); };
         if (M == 1) {

@@ -29,3 +29,15 @@ def test_lengths(eng, family, param, terms):
     for n0, f0, f1 in ((1, 3, 3000), (777, (1 << 20) + 1, (1 << 20) + 20000), (5, (1 << 40) - 30000, (1 << 40) + 30000)):
         job = ctd.CtdJob(family, 32, param, n0, n0 + terms, f0, f1)
         assert run(eng, job, 0) == run(eng, job, 1), (n0, f0)
+
+
+# class moduli on both sides of 32, where a block's targets change from an M-bit
+# reduction to the Shoup product: only lists this long give classes of 2560
+# terms and more with such moduli
+@pytest.mark.parametrize("family,param", [(O.PROTH, 3), (O.RIESEL, 12345), (O.MERSENNE, 0)])
+def test_long_lists(eng, family, param):
+    for f0, f1 in (((1 << 33) + 1, (1 << 33) + 8000), ((1 << 62) - 9000, (1 << 62) + 3000)):
+        job = ctd.CtdJob(family, 32, param, 11, 400011, f0, f1)
+        assert run(eng, job, 0) == run(eng, job, 1), f0
+    job = ctd.CtdJob(family, 512, param, 11, 300011, 101, 20000)
+    assert run(eng, job, 0) == run(eng, job, 1)
