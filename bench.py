@@ -101,23 +101,23 @@ PROTH_NCU = {"primes": 6047768,
              # warp instructions x active lanes per instruction, one entry per launch
              "thread_inst": {
                  "screen_kernel": 65171117 * 29.81,
-                 "classify_kernel_p0": 109554151 * 29.03,
-                 "classify_kernel_p1": 241305487 * 28.09,
-                 "classify_kernel_p2": 40675533 * 28.53,
-                 "classify_kernel_p3": 93172111 * 26.93,
-                 "classify_kernel_p4": 26558798 * 28.83,
-                 "classify_kernel_p5": 58077851 * 26.84,
-                 "classify_kernel_p6": 10047747 * 27.71,
-                 "classify_kernel_p7": 22809306 * 25.60,
-                 "refine_kernel": 245981681 * 26.61,
-                 "nine_kernel": 79744251 * 28.19,
+                 "classify_kernel_p0": 109552762 * 29.03,
+                 "classify_kernel_p1": 241294961 * 28.09,
+                 "classify_kernel_p2": 40679576 * 28.52,
+                 "classify_kernel_p3": 93172903 * 26.93,
+                 "classify_kernel_p4": 26558972 * 28.83,
+                 "classify_kernel_p5": 58073349 * 26.84,
+                 "classify_kernel_p6": 10046516 * 27.71,
+                 "classify_kernel_p7": 22806561 * 25.61,
+                 "refine_kernel": 245961704 * 26.61,
+                 "nine_kernel": 79746825 * 28.19,
                  "regroup_kernel": 56933014 * 15.98,
-                 "class_walk_kernel": 1368855968 * 26.09},
+                 "class_walk_kernel": 1064760657 * 29.81},
              # dram__bytes_read.sum + dram__bytes_write.sum of the same launches, MB
-             "dram_bytes": (62.127360 + 14.758912 + 55.779840 + 6.085888 + 64.821248 + 9.626880 + 31.815168 +
-                            1.307904 + 48.090112 + 3.739904 + 21.870336 + 0.407552 + 36.465152 + 1.719296 + 8.113152
-                            + 0.021248 + 15.670784 + 0.138752 + 83.027712 + 3.585792 + 68.413952 + 1.600256 +
-                            73.113856 + 11.770880 + 53.818624 + 3.506944) * 1e6}
+             "dram_bytes": (62.181120 + 14.798592 + 55.797760 + 6.120192 + 64.786688 + 9.624320 + 31.819264 +
+                            1.310976 + 48.071936 + 3.706112 + 21.867520 + 0.404736 + 36.450560 + 1.709568 + 8.111872
+                            + 0.019456 + 15.662592 + 0.133888 + 83.092224 + 3.571968 + 68.415232 + 1.509888 +
+                            73.121024 + 11.797504 + 53.845504 + 3.909632) * 1e6}
 SMARANDACHE_MULS_PER_UPDATE = (90 * 2 + 900 * 2.5) / 990
 TRIBONACCI_ALU_OPS_PER_UPDATE = 55 / 31
 
