@@ -658,6 +658,8 @@ static cudaError_t launch_ranks(const JobView &v, const uint64_t *d_primes, uint
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return e;
+    if (!list.cap)  // no list: the tiles have finished their primes and pushed all hits
+        return cudaSuccess;
     note_kernel_launch();
     const uint64_t blocks = ((list.cap < n ? list.cap : n) + 255) / 256;
     rank_finish_kernel<FAM><<<(unsigned)(blocks < grid ? blocks : grid), 256, 0, st>>>(v, list);

@@ -3306,13 +3306,14 @@ int launch_residues(const JobView &view, const uint64_t *d_primes, uint64_t npri
             return rc0;
         const uint32_t cap = rank_list_cap(nprimes);
         if (cap > scratch->rank_cap) {
-            cudaFree(scratch->rank_items);
-            scratch->rank_items = nullptr;
-            scratch->rank_cap = 0;
-            if (cudaMalloc(&scratch->rank_items, cap * sizeof(RankItem) + RANK_HEAVY * sizeof(RankHits)) == cudaSuccess)
+            void *grown = nullptr;
+            if (cudaMalloc(&grown, cap * sizeof(RankItem) + RANK_HEAVY * sizeof(RankHits)) == cudaSuccess) {
+                cudaFree(scratch->rank_items);
+                scratch->rank_items = grown;
                 scratch->rank_cap = cap;
-            else  // the tiles finish their primes themselves
+            } else {  // the tiles finish the primes that the present list, if any, has no room for
                 (void)cudaGetLastError();
+            }
         }
         RankItem *const items = (RankItem *)scratch->rank_items;
         const RankList list{items, &scratch->counters->nrefine, scratch->rank_cap,
