@@ -3304,8 +3304,13 @@ int launch_residues(const JobView &view, const uint64_t *d_primes, uint64_t npri
         const int rc0 = ensure_class_scratch(scratch, 0, err);  // its counters
         if (rc0)
             return rc0;
+        // Into a graph the launch goes without the list, and the tiles finish
+        // their primes themselves: nothing may be allocated during a capture,
+        // and a later, longer list would free the memory that the graph writes.
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        const bool plain = cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
         const uint32_t cap = rank_list_cap(nprimes);
-        if (cap > scratch->rank_cap) {
+        if (plain && cap > scratch->rank_cap) {
             void *grown = nullptr;
             if (cudaMalloc(&grown, cap * sizeof(RankItem) + RANK_HEAVY * sizeof(RankHits)) == cudaSuccess) {
                 cudaFree(scratch->rank_items);
@@ -3316,9 +3321,9 @@ int launch_residues(const JobView &view, const uint64_t *d_primes, uint64_t npri
             }
         }
         RankItem *const items = (RankItem *)scratch->rank_items;
-        const RankList list{items, &scratch->counters->nrefine, scratch->rank_cap,
-                            (RankHits *)(items + scratch->rank_cap), &scratch->counters->nnine,
-                            scratch->rank_cap ? RANK_HEAVY : 0u};
+        const uint32_t room = plain ? scratch->rank_cap : 0;
+        const RankList list{items, &scratch->counters->nrefine, room, (RankHits *)(items + scratch->rank_cap),
+                            &scratch->counters->nnine, room ? RANK_HEAVY : 0u};
         cudaError_t rc;
         if (view.family == FIBONACCI)
             rc = launch_ranks<FIBONACCI>(view, d_primes, nprimes, scratch->sm_count, stream, scratch->counters, list);
