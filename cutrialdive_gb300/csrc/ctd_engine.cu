@@ -890,7 +890,6 @@ int ctd_run_plain(ctd_ctx *ctx, const ctd_job *job, uint32_t *counts_inout, uint
     if (rc)
         return rc;
     JobView view = make_view(job, ctx->d_counts, ctx->d_factors);
-    view.dense = 1;
     std::string err;
 
     uint64_t f0 = resume_after_prime ? resume_after_prime + 1 : job->f0;
@@ -926,6 +925,7 @@ int ctd_run_plain(ctd_ctx *ctx, const ctd_job *job, uint32_t *counts_inout, uint
             view.variant = variant_of(ctx, job->family, bits);
             view.classify_min = classify_min_of(ctx, job->family, bits);
             view.refine_q = refine_q_of(ctx, job->family, bits);
+            view.list = fy <= 1ull << 62 ? LIST_DENSE : fx >= 1ull << 63 ? LIST_WIDE : LIST_ANY;
             choose_tiles(ctx, job->family, bits, np, N, grid, block, view.tiles, view.tile_len);
             rc = launch_residues(view, ctx->d_primes, np, grid, block, st, err, ctx->rs);
             if (rc)

@@ -37,6 +37,18 @@ struct FactorsView {
     uint32_t max_factors;
 };
 
+// What a launch's list is known to hold, for the choice of ranks and orders.
+// Their tiles take primes below 2^62; beyond it the orders of 2 are found prime
+// by prime.  From 2^62 to 2^63 classes are better than that (the 390,000 primes
+// of a 2^24-wide range at 2^62, n = 1..1000000: 52 ms by orders, 3 by classes),
+// from 2^63 on, where classes are not taken and every term is walked, the
+// orders are (at 2^63: 40 ms, the walk 168).
+enum : uint32_t {
+    LIST_ANY = 0,    // any primes in any order
+    LIST_DENSE = 1,  // every prime of a range that ends at 2^62 at most
+    LIST_WIDE = 2,   // every prime of a range that starts at 2^63 or later
+};
+
 // What a residue launch needs to know about its job.
 struct JobView {
     uint32_t family;
@@ -44,7 +56,7 @@ struct JobView {
     uint32_t variant;    // step form (CTD_VARIANT_*)
     uint32_t classify_min;  // doubling families: index ranges this long or longer walk power-residue classes
     uint32_t refine_q;   // largest rare prime whose character refines the classes (0: 61; < 11: none)
-    uint32_t dense;      // the launch's list holds every prime of its range
+    uint32_t list;       // LIST_*
     uint64_t param;      // k, n or base
     uint64_t n0, n1;     // index range of the factors buffer
     uint64_t tile_len;   // indices per tile (last tile may be shorter)

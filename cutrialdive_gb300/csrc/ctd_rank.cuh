@@ -625,7 +625,7 @@ __global__ void __launch_bounds__(256) rank_heavy_kernel(JobView job, RankList l
 // whether a job's primes go by tiles of ranks
 inline bool takes_ranks(const JobView &v)
 {
-    const bool mersenne = v.family == MERSENNE && v.dense;
+    const bool mersenne = v.family == MERSENNE && v.list != LIST_ANY;
     return (v.family == FIBONACCI || v.family == LUCAS || mersenne) && v.variant == CTD_VARIANT_AUTO && v.n0 >= 1 &&
            v.n1 <= TRIAL_LIMIT && v.n1 - v.n0 >= (mersenne ? order_min_terms(v.n1) : rank_min_terms(v.n1));
 }
