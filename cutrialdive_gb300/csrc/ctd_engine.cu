@@ -845,6 +845,7 @@ int ctd_residues_device(ctd_ctx *ctx, const ctd_job *job, const uint64_t *d_prim
     v.variant = variant_of(ctx, job->family, bits);
     v.classify_min = classify_min_of(ctx, job->family, bits);
     v.refine_q = refine_q_of(ctx, job->family, bits);
+    v.list = job->f0 >= 1ull << 62 ? LIST_HIGH : LIST_ANY;
     const int block = default_block(ctx, job->family, bits);
     const int grid = default_grid(ctx, job->family, block, bits);
     choose_tiles(ctx, job->family, bits, nprimes, job->n1 - job->n0, grid, block, v.tiles, v.tile_len);
@@ -925,7 +926,10 @@ int ctd_run_plain(ctd_ctx *ctx, const ctd_job *job, uint32_t *counts_inout, uint
             view.variant = variant_of(ctx, job->family, bits);
             view.classify_min = classify_min_of(ctx, job->family, bits);
             view.refine_q = refine_q_of(ctx, job->family, bits);
-            view.list = fy <= 1ull << 62 ? LIST_DENSE : fx >= 1ull << 63 ? LIST_WIDE : LIST_ANY;
+            view.list = fy <= 1ull << 62   ? LIST_DENSE
+                        : fx >= 1ull << 63 ? LIST_WIDE
+                        : fx >= 1ull << 62 ? LIST_HIGH
+                                           : LIST_ANY;
             choose_tiles(ctx, job->family, bits, np, N, grid, block, view.tiles, view.tile_len);
             rc = launch_residues(view, ctx->d_primes, np, grid, block, st, err, ctx->rs);
             if (rc)

@@ -46,7 +46,8 @@ struct FactorsView {
 enum : uint32_t {
     LIST_ANY = 0,    // any primes in any order
     LIST_DENSE = 1,  // every prime of a range that ends at 2^62 at most
-    LIST_WIDE = 2,   // every prime of a range that starts at 2^63 or later
+    LIST_HIGH = 2,   // primes of 2^62 and more
+    LIST_WIDE = 3,   // every prime of a range that starts at 2^63 or later
 };
 
 // What a residue launch needs to know about its job.
@@ -128,7 +129,7 @@ struct ClassCounters {
     uint32_t fill[CLASS_BUCKETS];   // regroup cursors
     unsigned long long next;        // walk work counter
     uint32_t nrefine;               // primes listed for the rare-prime refinement (for their rank: Fibonacci, Lucas)
-    uint32_t nlisted[8];            // primes the screen left for classification, by divisibility pattern
+    uint32_t nlisted[8];            // primes the screen left for classification, by divisibility pattern ([0]: ranks, the list's sparse tiles)
     uint32_t wide;                  // a prime of the launch is 2^40 or above
     uint32_t nnine;                 // primes listed for the 9th-power character (for their many hits: ranks)
 };

@@ -266,6 +266,12 @@ struct RankShared {
     uint32_t flags;              // 1: an even or repeated entry, or one beyond 2^62
 };
 
+// whether a tile's primes, all odd or not, fit its bitmap
+__device__ __forceinline__ bool rank_fits(bool odd, uint64_t lo, uint64_t hi)
+{
+    return odd && lo >= 3 && hi < (1ull << 62) && hi - lo <= 2 * (RANK_SPAN - 2);
+}
+
 // one tile of n <= RANK_TILE primes of the list; false when it does not fit
 // the bitmap (a sparse or unordered list), and nothing was pushed
 template <uint32_t FAM, bool NARROW>
@@ -309,7 +315,7 @@ __device__ bool rank_tile(const JobView &job, const RankList &list, RankShared &
     }
     __syncthreads();
     const uint64_t lo = sh.lo, hi = sh.hi;
-    if (sh.flags || lo < 3 || hi >= (1ull << 62) || hi - lo > 2 * (RANK_SPAN - 2))
+    if (!rank_fits(!sh.flags, lo, hi))
         return false;
     const uint64_t m0 = lo - 1;                              // even; D = m0 + 2 i
     const uint32_t span = (uint32_t)((hi - lo) >> 1) + 2;    // i < span <= RANK_SPAN
@@ -558,6 +564,57 @@ __device__ __noinline__ void rank_alone(const JobView &job, const RankList &list
     }
 }
 
+// A list that may hold any primes is looked over first: sparse counts its tiles
+// that do not fit the bitmap.  Such a tile is walked item by item in
+// rank_kernel, by two or three times the time that the same items take in a
+// grid of their own (one prime in three of a 2^26-wide range at 2^33:
+// n = 1..50000, 10.6 ms and 5.0; n = 1..200000, 17.0 and 5.6), while a tile that
+// fits takes an eighth of it.  So a list with more than a quarter of sparse
+// tiles goes to rank_walk_kernel.  (sparse null: a dense list.)
+__device__ __forceinline__ bool rank_sparse(const uint32_t *sparse, uint64_t nprimes, uint32_t tile)
+{
+    return sparse && 4ull * *sparse > (nprimes + tile - 1) / tile;
+}
+
+// a warp a tile; bound by reading the list once
+__global__ void __launch_bounds__(256) rank_fit_kernel(const uint64_t *__restrict__ primes, uint64_t nprimes,
+                                                       uint32_t tile, uint32_t *sparse)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t ntiles = (nprimes + tile - 1) / tile;
+    uint32_t count = 0;
+    for (uint64_t t = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5); t < ntiles; t += (uint64_t)gridDim.x * 8) {
+        const uint64_t *const p = primes + t * tile;
+        const uint32_t n = (uint32_t)(nprimes - t * tile < tile ? nprimes - t * tile : tile);
+        uint64_t lo = ~0ull, hi = 0;
+        bool fits = true;
+        for (uint32_t i = lane; i < n; i += 32) {
+            const uint64_t x = p[i];
+            lo = x < lo ? x : lo;
+            hi = x > hi ? x : hi;
+            fits &= (x & 1) && !(i + 1 < n && p[i + 1] == x);  // a repeat fills its mark twice
+        }
+        for (int o = 16; o; o >>= 1) {
+            const uint64_t l = __shfl_xor_sync(0xffffffffu, lo, o), h = __shfl_xor_sync(0xffffffffu, hi, o);
+            lo = l < lo ? l : lo;
+            hi = h > hi ? h : hi;
+        }
+        count += !rank_fits(__all_sync(0xffffffffu, fits), lo, hi);
+    }
+    if (lane == 0 && count)
+        atomicAdd(sparse, count);
+}
+
+// the walk, item by item, of a list that is too sparse for tiles
+template <uint32_t FAM>
+__global__ void __launch_bounds__(256, min_ctas_per_sm(FAM))
+rank_walk_kernel(JobView job, const uint64_t *__restrict__ primes, uint64_t nprimes, uint32_t tile,
+                 unsigned long long *next, const uint32_t *sparse)
+{
+    if (rank_sparse(sparse, nprimes, tile))
+        residue_items<FAM>(job, primes, nprimes, next);
+}
+
 // Bound by integer issue (56 % of the slots, 20 of 32 lanes): the powers, about
 // 20 bits of two narrow Montgomery products each, are the largest part, then
 // the marks and the primes' multiples.  A tile of 1024 primes shares one walk
@@ -568,8 +625,10 @@ __device__ __noinline__ void rank_alone(const JobView &job, const RankList &list
 template <uint32_t FAM>
 __global__ void __launch_bounds__(256, RANK_CTAS)
 rank_kernel(JobView job, const uint64_t *__restrict__ primes, uint64_t nprimes, uint32_t tile, unsigned long long *next,
-            RankList list)
+            const uint32_t *sparse, RankList list)
 {
+    if (rank_sparse(sparse, nprimes, tile))
+        return;
     extern __shared__ __align__(16) unsigned char rank_smem[];
     RankShared &sh = *reinterpret_cast<RankShared *>(rank_smem);
     const uint64_t ntiles = (nprimes + tile - 1) / tile;
@@ -625,8 +684,9 @@ __global__ void __launch_bounds__(256) rank_heavy_kernel(JobView job, RankList l
 // whether a job's primes go by tiles of ranks
 inline bool takes_ranks(const JobView &v)
 {
-    const bool mersenne = v.family == MERSENNE && v.list != LIST_ANY;
-    return (v.family == FIBONACCI || v.family == LUCAS || mersenne) && v.variant == CTD_VARIANT_AUTO && v.n0 >= 1 &&
+    const bool mersenne = v.family == MERSENNE && (v.list == LIST_DENSE || v.list == LIST_WIDE);
+    const bool ranks = (v.family == FIBONACCI || v.family == LUCAS) && v.list <= LIST_DENSE;
+    return (ranks || mersenne) && v.variant == CTD_VARIANT_AUTO && v.n0 >= 1 &&
            v.n1 <= TRIAL_LIMIT && v.n1 - v.n0 >= (mersenne ? order_min_terms(v.n1) : rank_min_terms(v.n1));
 }
 
@@ -640,8 +700,8 @@ static uint32_t rank_list_cap(uint64_t nprimes)
 }
 
 template <uint32_t FAM>
-static cudaError_t launch_ranks(const JobView &v, const uint64_t *d_primes, uint64_t n, int sm_count, cudaStream_t st,
-                                ClassCounters *counters, const RankList &list)
+static cudaError_t launch_ranks(const JobView &v, const uint64_t *d_primes, uint64_t n, int sm_count, int walk_grid,
+                                int walk_block, cudaStream_t st, ClassCounters *counters, const RankList &list)
 {
     cudaError_t e = allow_smem(rank_kernel<FAM>, sizeof(RankShared));
     if (e == cudaSuccess)
@@ -653,11 +713,40 @@ static cudaError_t launch_ranks(const JobView &v, const uint64_t *d_primes, uint
     const uint64_t per = (n + grid - 1) / grid;
     const uint32_t tile = per < RANK_TILE ? (uint32_t)per : RANK_TILE;
     const uint64_t ntiles = (n + tile - 1) / tile;
+    const bool any = FAM != MERSENNE && v.list == LIST_ANY;
+    // The primes of sparse tiles: each by one rank for the whole index range,
+    // where there are threads' worth of them or a long range makes up for its
+    // latency (0.65 ms for n = 1..50000, however few the primes).  n = 1..50000,
+    // 584,000 primes around 2^34: 4.1 ms in index tiles, 2.0 whole; 29,000 at
+    // 2^33: 0.38 and 0.67.
+    JobView w = v;
+    const uint64_t threads = (uint64_t)walk_grid * walk_block;
+    if (any && fibonacci_rank_pays(v.n0, v.n1) && (n >= threads || (4 * n >= threads && v.n1 >= 1u << 14))) {
+        w.tiles = 1;
+        w.tile_len = v.n1 - v.n0;
+    }
+    uint32_t *const sparse = any ? &counters->nlisted[0] : nullptr;
+    if (any) {
+        const uint64_t blocks = (ntiles + 7) / 8;
+        rank_fit_kernel<<<(unsigned)(blocks < grid ? blocks : grid), 256, 0, st>>>(d_primes, n, tile, sparse);
+        e = cudaGetLastError();
+        if (e != cudaSuccess)
+            return e;
+        note_kernel_launch();
+    }
     rank_kernel<FAM><<<(unsigned)(ntiles < grid ? ntiles : grid), 256, sizeof(RankShared), st>>>(
-        v, d_primes, n, tile, &counters->next, list);
+        w, d_primes, n, tile, &counters->next, sparse, list);
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return e;
+    if constexpr (FAM != MERSENNE)
+        if (any) {
+            note_kernel_launch();
+            rank_walk_kernel<FAM><<<walk_grid, walk_block, 0, st>>>(w, d_primes, n, tile, &counters->next, sparse);
+            e = cudaGetLastError();
+            if (e != cudaSuccess)
+                return e;
+        }
     if (!list.cap)  // no list: the tiles have finished their primes and pushed all hits
         return cudaSuccess;
     note_kernel_launch();

@@ -1090,6 +1090,15 @@ __device__ void run_fibonacci_rank(const JobView &job, uint64_t p, uint64_t s, u
         push(job.fb, n - job.n0, p);
 }
 
+// Whether the terms s .. e - 1 of one prime go by its rank: measured on a
+// GB300, a table prime of that path costs about 3.9 terms of the walk: taken
+// when e - s > 3.9 pi(e), with pi(e) ~ e / ln e and ln e ~ 0.69 floor(log2 e),
+// i.e. (e - s) floor(log2 e) > 6 e (+4096 for its fixed cost)
+CTD_HD bool fibonacci_rank_pays(uint64_t s, uint64_t e)
+{
+    return e <= TRIAL_LIMIT && (e - s) * (uint64_t)(63 - clz64(e)) > 6 * e + 4096;
+}
+
 // Fibonacci / Lucas: state (S(n-1), S(n)), one addmod per step
 // (fibonacci.hpp:245-285, lucas.hpp:394-418).  The reference's
 // make_state(0) leaves S(-1) = 0 and S(0) = 0, so a job starting at n0 = 0
@@ -1098,12 +1107,8 @@ __device__ void run_fibonacci_rank(const JobView &job, uint64_t p, uint64_t s, u
 template <uint32_t FAM>
 __device__ __forceinline__ void run_fibonacci(const JobView &job, uint64_t p, uint64_t s, uint64_t e)
 {
-    // measured on a GB300, a table prime of the rank-of-apparition path costs
-    // about 3.9 terms of the walk: taken when e - s > 3.9 pi(e), with pi(e) ~
-    // e / ln e and ln e ~ 0.69 floor(log2 e), i.e. (e - s) floor(log2 e) >
-    // 6 e (+4096 for its fixed cost)
-    if (job.n0 != 0 && s != 0 && (p & 1) && p != 5 && p < (1ull << 62) && e <= TRIAL_LIMIT &&
-        (e - s) * (uint64_t)(63 - __clzll(e)) > 6 * e + 4096 && job.variant != CTD_VARIANT_WALK) {
+    if (job.n0 != 0 && s != 0 && (p & 1) && p != 5 && p < (1ull << 62) && fibonacci_rank_pays(s, e) &&
+        job.variant != CTD_VARIANT_WALK) {
         run_fibonacci_rank<FAM>(job, p, s, e);
         return;
     }
@@ -2126,8 +2131,8 @@ __device__ __forceinline__ void residue_item(const JobView &job, const uint64_t 
 // every SM finishes within one item of the others; without one, threads
 // stride over the items.
 template <uint32_t FAM>
-__global__ void __launch_bounds__(256, min_ctas_per_sm(FAM))
-residue_kernel(JobView job, const uint64_t *__restrict__ primes, uint64_t nprimes, unsigned long long *next)
+__device__ __forceinline__ void residue_items(const JobView &job, const uint64_t *__restrict__ primes, uint64_t nprimes,
+                                              unsigned long long *next)
 {
     const uint64_t items = nprimes * job.tiles;
     if (!next) {
@@ -2147,6 +2152,12 @@ residue_kernel(JobView job, const uint64_t *__restrict__ primes, uint64_t nprime
         if (base + lane < items)
             residue_item<FAM>(job, primes, nprimes, base + lane);
     }
+}
+template <uint32_t FAM>
+__global__ void __launch_bounds__(256, min_ctas_per_sm(FAM))
+residue_kernel(JobView job, const uint64_t *__restrict__ primes, uint64_t nprimes, unsigned long long *next)
+{
+    residue_items<FAM>(job, primes, nprimes, next);
 }
 
 // ------------------------------------------ classified doubling launches
@@ -3326,11 +3337,11 @@ int launch_residues(const JobView &view, const uint64_t *d_primes, uint64_t npri
                             &scratch->counters->nnine, room ? RANK_HEAVY : 0u};
         cudaError_t rc;
         if (view.family == FIBONACCI)
-            rc = launch_ranks<FIBONACCI>(view, d_primes, nprimes, scratch->sm_count, stream, scratch->counters, list);
+            rc = launch_ranks<FIBONACCI>(view, d_primes, nprimes, scratch->sm_count, grid, block, stream, scratch->counters, list);
         else if (view.family == LUCAS)
-            rc = launch_ranks<LUCAS>(view, d_primes, nprimes, scratch->sm_count, stream, scratch->counters, list);
+            rc = launch_ranks<LUCAS>(view, d_primes, nprimes, scratch->sm_count, grid, block, stream, scratch->counters, list);
         else
-            rc = launch_ranks<MERSENNE>(view, d_primes, nprimes, scratch->sm_count, stream, scratch->counters, list);
+            rc = launch_ranks<MERSENNE>(view, d_primes, nprimes, scratch->sm_count, grid, block, stream, scratch->counters, list);
         if (rc != cudaSuccess) {
             err = std::string("rank kernel launch: ") + cudaGetErrorString(rc);
             return CTD_ERR_CUDA;
