@@ -450,16 +450,19 @@ static int ensure_windows(SieveWorkspace *ws, uint64_t nwin, std::string &err)
     return CTD_OK;
 }
 
-static int ensure_starts(SieveWorkspace *ws, std::string &err)
+// room for a start a base prime; without the memory for it (8 bytes each) the
+// windows divide for themselves
+static void ensure_starts(SieveWorkspace *ws)
 {
-    if (ws->nbase > ws->starts_cap) {
-        cudaFree(ws->d_starts);
-        ws->d_starts = nullptr;
-        ws->starts_cap = 0;
-        CUDA_TRY(cudaMalloc(&ws->d_starts, ws->nbase * sizeof(SieveStart)));
+    if (ws->nbase <= ws->starts_cap)
+        return;
+    cudaFree(ws->d_starts);
+    ws->d_starts = nullptr;
+    ws->starts_cap = 0;
+    if (cudaMalloc(&ws->d_starts, ws->nbase * sizeof(SieveStart)) == cudaSuccess)
         ws->starts_cap = ws->nbase;
-    }
-    return CTD_OK;
+    else
+        (void)cudaGetLastError();
 }
 
 // Launches the passes over the odd numbers lo_odd .. lo_odd + 2 (nodd - 1),
@@ -532,12 +535,10 @@ static int sieve_odd(SieveWorkspace *ws, uint64_t lo_odd, uint64_t nodd, const u
     int rc = ensure_windows(ws, nwin, err);
     if (rc)
         return rc;
-    rc = ensure_starts(ws, err);
-    if (rc)
-        return rc;
+    ensure_starts(ws);
     uint32_t chunks = 0;
-    rc = launch_sieve<T>(lo_odd, nodd, d_base, nbase, ws->d_starts, ws->d_bits, ws->d_wcount, ws->d_offsets,
-                         ws->sm_count, d_out, capacity, out_base, &chunks, st, err);
+    rc = launch_sieve<T>(lo_odd, nodd, d_base, nbase, nbase <= ws->starts_cap ? ws->d_starts : nullptr, ws->d_bits,
+                         ws->d_wcount, ws->d_offsets, ws->sm_count, d_out, capacity, out_base, &chunks, st, err);
     if (rc)
         return rc;
     CUDA_TRY(cudaMemcpyAsync(ws->h_total, ws->d_offsets + chunks, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
@@ -644,7 +645,9 @@ int sieve_prepare_base(SieveWorkspace *ws, uint64_t hi, cudaStream_t st, std::st
     if (hi < 3)
         return CTD_OK;
     const int rc = ensure_base(ws, isqrt64(hi - 1), st, err);
-    return rc ? rc : ensure_starts(ws, err);
+    if (!rc)
+        ensure_starts(ws);
+    return rc;
 }
 
 int sieve_prepare_windows(SieveWorkspace *ws, uint64_t max_width, std::string &err)
@@ -674,7 +677,7 @@ int sieve_odd_async(SieveWorkspace *ws, uint64_t lo, uint64_t hi, uint64_t *d_ou
     const uint64_t lo_odd = lo < 3 ? 3 : (lo | 1);
     const uint64_t nodd = lo_odd < hi ? (hi - lo_odd + 1) / 2 : 0;
     const uint64_t nwin = nodd ? (nodd + WIN_ODD - 1) / WIN_ODD : 0;
-    if (nwin > ws->win_cap || !ws->d_base || ws->nbase > ws->starts_cap) {
+    if (nwin > ws->win_cap || !ws->d_base) {
         err = "sieve scratch not prepared for this segment";
         return CTD_ERR_INVALID_ARGUMENT;
     }
@@ -684,7 +687,8 @@ int sieve_odd_async(SieveWorkspace *ws, uint64_t lo, uint64_t hi, uint64_t *d_ou
         return CTD_OK;
     }
     uint32_t chunks = 0;
-    const int rc = launch_sieve<uint64_t>(lo_odd, nodd, ws->d_base, ws->nbase, ws->d_starts, ws->d_bits, ws->d_wcount,
+    const int rc = launch_sieve<uint64_t>(lo_odd, nodd, ws->d_base, ws->nbase,
+                                          ws->nbase <= ws->starts_cap ? ws->d_starts : nullptr, ws->d_bits, ws->d_wcount,
                                           ws->d_offsets, ws->sm_count, d_out, capacity, 0, &chunks, st, err);
     *count_out = ws->d_offsets + chunks;
     return rc;
