@@ -371,6 +371,14 @@ uint64_t default_segment(const ctd_ctx *ctx, uint32_t family, int bits, uint64_t
     return longer;
 }
 
+// the list of every prime of [lo, hi)
+uint32_t list_of_range(uint64_t lo, uint64_t hi)
+{
+    if (hi <= 1ull << 62)
+        return LIST_DENSE;
+    return lo >= 1ull << 63 ? LIST_WIDE : lo >= 1ull << 62 ? LIST_HIGH : LIST_ANY;
+}
+
 JobView make_view(const ctd_job *job, uint32_t *d_counts, uint64_t *d_factors)
 {
     JobView v{};
@@ -613,7 +621,10 @@ int ctd_autotune(ctd_ctx *ctx, const ctd_job *job, double budget_s, ctd_tuning *
     cudaEvent_t ea, eb;
     CTX_CUDA(cudaEventCreate(&ea));
     CTX_CUDA(cudaEventCreate(&eb));
+    // (what is timed is what ctd_run_plain launches for these primes)
     JobView view = make_view(job, ctx->d_counts, ctx->d_factors);
+    view.list = list_of_range(fx, fy);
+    const bool ranks = residues_by_ranks(view);
     // milliseconds of one residue launch over `n` sample primes (best of two
     // after a warm-up); the counts are cleared so no term overflows
     auto time_config = [&](const ctd_tuning &c, uint64_t n, float &ms) -> int {
@@ -667,8 +678,9 @@ int ctd_autotune(ctd_ctx *ctx, const ctd_job *job, double budget_s, ctd_tuning *
     const uint32_t fam = job->family;
     // power-residue classes (doubling families): always, or never; then the
     // rare primes of their refinement: all (up to 127, the starting entry),
-    // none, up to 31
-    if (!rc && (fam == CTD_PROTH || fam == CTD_RIESEL || fam == CTD_MERSENNE)) {
+    // none, up to 31.  (Ranks and orders take neither classes nor a launch
+    // shape nor index tiles: no trial of them could tell more than noise.)
+    if (!rc && !ranks && (fam == CTD_PROTH || fam == CTD_RIESEL || fam == CTD_MERSENNE)) {
         for (uint32_t cm : {1u, 0xffffffffu}) {
             if (elapsed() >= budget_s)
                 break;
@@ -688,7 +700,7 @@ int ctd_autotune(ctd_ctx *ctx, const ctd_job *job, double budget_s, ctd_tuning *
     }
     // launch shape: block size and resident CTAs per SM
     const int blocks[] = {256, 128, 64};
-    for (int bi = 0; !rc && bi < 3 && elapsed() < budget_s; ++bi) {
+    for (int bi = 0; !rc && !ranks && bi < 3 && elapsed() < budget_s; ++bi) {
         const int occ = residue_blocks_per_sm(fam, blocks[bi]);
         const int cands[] = {occ, occ - 1, occ / 2, (occ * 3) / 4};
         for (int ci = 0; !rc && ci < 4 && elapsed() < budget_s; ++ci) {
@@ -713,7 +725,7 @@ int ctd_autotune(ctd_ctx *ctx, const ctd_job *job, double budget_s, ctd_tuning *
         tiles_for(np, N, wgrid, winner.block_size, winner.items_per_thread, winner.min_tile, tt, tl);
         seen_tiles[nseen++] = tt;
     }
-    for (int i = 0; !rc && i < 5 && elapsed() < budget_s; ++i)
+    for (int i = 0; !rc && !ranks && i < 5 && elapsed() < budget_s; ++i)
         for (int j = 0; !rc && j < 5 && elapsed() < budget_s; ++j) {
             ctd_tuning t = winner;
             t.items_per_thread = items[i];
@@ -756,6 +768,7 @@ int ctd_autotune(ctd_ctx *ctx, const ctd_job *job, double budget_s, ctd_tuning *
             view.variant = winner.variant;
             view.classify_min = winner.classify_min ? winner.classify_min : DEFAULT_CLASSIFY_MIN;
             view.refine_q = winner.refine_q;
+            view.list = list_of_range(fx, sy);
             uint64_t n = 0;
             float t = 0;
             if (cudaMemsetAsync(ctx->d_counts, 0, N * sizeof(uint32_t), st) != cudaSuccess)
@@ -926,10 +939,7 @@ int ctd_run_plain(ctd_ctx *ctx, const ctd_job *job, uint32_t *counts_inout, uint
             view.variant = variant_of(ctx, job->family, bits);
             view.classify_min = classify_min_of(ctx, job->family, bits);
             view.refine_q = refine_q_of(ctx, job->family, bits);
-            view.list = fy <= 1ull << 62   ? LIST_DENSE
-                        : fx >= 1ull << 63 ? LIST_WIDE
-                        : fx >= 1ull << 62 ? LIST_HIGH
-                                           : LIST_ANY;
+            view.list = list_of_range(fx, fy);
             choose_tiles(ctx, job->family, bits, np, N, grid, block, view.tiles, view.tile_len);
             rc = launch_residues(view, ctx->d_primes, np, grid, block, st, err, ctx->rs);
             if (rc)

@@ -166,6 +166,9 @@ int prepare_residue_tables(int device, std::string &err);
 // long ranges go through the classified launches (classify, regroup, walk).
 int launch_residues(const JobView &view, const uint64_t *d_primes, uint64_t nprimes, int grid, int block,
                     cudaStream_t stream, std::string &err, ResidueScratch *scratch = nullptr);
+// Whether launch_residues, with a scratch, takes this view by ranks or orders:
+// launch shape and index tiles then have no effect.
+bool residues_by_ranks(const JobView &view);
 // One job of a batched launch: its view (factors buffer, index range,
 // tiles), its odd-prime range [f0, f1) and whether it walks power-residue
 // classes (doubling families over long ranges).

@@ -3306,6 +3306,8 @@ static int launch_classified(const JobView &v, const uint64_t *d_primes, uint64_
     return CTD_OK;
 }
 
+bool residues_by_ranks(const JobView &view) { return takes_ranks(view); }
+
 int launch_residues(const JobView &view, const uint64_t *d_primes, uint64_t nprimes, int grid, int block,
                     cudaStream_t stream, std::string &err, ResidueScratch *scratch)
 {
