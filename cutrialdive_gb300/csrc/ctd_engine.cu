@@ -713,9 +713,10 @@ int ctd_autotune(ctd_ctx *ctx, const ctd_job *job, double budget_s, ctd_tuning *
             rc = try_config(t, winner, best_ms);
         }
     }
-    // tiling: only where it changes the split of this sample
-    const uint32_t items[] = {2, 4, 8, 16, 32};
-    const uint32_t tiles_min[] = {1024, 2048, 4096, 8192, 16384};
+    // tiling: only where it changes the split of this sample.  First the tiles
+    // that an untuned context gives a list shorter than its threads
+    const uint32_t items[] = {1, 2, 4, 8, 16, 32};
+    const uint32_t tiles_min[] = {short_list_tile(fam), 1024, 2048, 4096, 8192, 16384};
     const int wgrid = grid_for(ctx, fam, winner.block_size, winner.ctas_per_sm);
     uint32_t seen_tiles[32];
     int nseen = 0;
@@ -725,8 +726,10 @@ int ctd_autotune(ctd_ctx *ctx, const ctd_job *job, double budget_s, ctd_tuning *
         tiles_for(np, N, wgrid, winner.block_size, winner.items_per_thread, winner.min_tile, tt, tl);
         seen_tiles[nseen++] = tt;
     }
-    for (int i = 0; !rc && !ranks && i < 5 && elapsed() < budget_s; ++i)
-        for (int j = 0; !rc && j < 5 && elapsed() < budget_s; ++j) {
+    for (int i = 0; !rc && !ranks && i < 6 && elapsed() < budget_s; ++i)
+        for (int j = 0; !rc && j < 6 && elapsed() < budget_s; ++j) {
+            if ((i == 0) != (j == 0) || !tiles_min[j])
+                continue;
             ctd_tuning t = winner;
             t.items_per_thread = items[i];
             t.min_tile = tiles_min[j];
