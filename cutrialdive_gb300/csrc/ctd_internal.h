@@ -56,7 +56,7 @@ struct JobView {
     uint32_t tiles;      // index tiles per prime (>= 1)
     uint32_t variant;    // step form (CTD_VARIANT_*)
     uint32_t classify_min;  // doubling families: index ranges this long or longer walk power-residue classes
-    uint32_t refine_q;   // largest rare prime whose character refines the classes (0: 61; < 11: none)
+    uint32_t refine_q;   // largest rare prime whose character refines the classes (0: 127; < 11: none)
     uint32_t list;       // LIST_*
     uint64_t param;      // k, n or base
     uint64_t n0, n1;     // index range of the factors buffer
@@ -150,7 +150,8 @@ struct ResidueScratch {
     uint32_t *nine = nullptr;    // indices of the primes for the 9th-power character
     uint64_t cap = 0;  // primes
     ClassCounters *counters = nullptr;
-    void *rank_items = nullptr;  // Fibonacci, Lucas: primes whose rank is left to take (RankItem), then those with many hits (RankHits)
+    // Fibonacci, Lucas, Mersenne: the primes whose rank is left to take (RankItem), then those with many hits (RankHits)
+    void *rank_items = nullptr;
     uint32_t rank_cap = 0;
 };
 ResidueScratch *residue_scratch_create(int device, int sm_count);

@@ -12,7 +12,7 @@
 // For the powers of 2 the same holds with the 2^u-th roots (2^u | p - 1):
 // z = 2^-((p-1)/2^u) has order 2^i, y must lie in the subgroup of order 2^i
 // (y^(2^i) = 1), and n is fixed mod 2^i by a discrete logarithm in that
-// cyclic 2-group (a scan of its at most 8 elements).  The conditions are
+// cyclic 2-group (of at most 4 elements, see two_part).  The conditions are
 // necessary, never sufficient: the walk still tests every n of the class
 // exactly, so the hits are exactly the walk's (no hit is lost: an n outside
 // the class cannot satisfy z^n = y).  Over random primes the class keeps
@@ -30,7 +30,8 @@
 
 namespace ctd {
 
-// largest power of 2 taken from p - 1 (2^3 = 8 classes at most: the
+// largest power of 2 taken from p - 1 (4 classes at most, as 2 is a square
+// where 8 divides p - 1: the
 // higher 2-power characters would shave about 3 % more terms for twice the
 // set-up)
 constexpr int POWRES_MAX_2EXP = 3;

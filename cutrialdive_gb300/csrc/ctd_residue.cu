@@ -642,12 +642,14 @@ __device__ __forceinline__ void run_doubling(const JobView &job, uint64_t p, uin
 // ------------------------------------- doubling over power-residue classes
 // For long index ranges the doubling families first classify each prime
 // (ctd_powres.cuh): every zero n of k*2^n-+1 (2^n-1) mod p satisfies
-// n = r (mod M) for a class M | 2^3 * 3 * 5 * 7 read off the 2-power, 3rd,
-// 5th and 7th power residues of 2 and of the target, and about 40 % of the
+// n = r (mod M) for a class M | 2^2 * 3 * 5 * 7 read off the 2-power, 3rd,
+// 5th and 7th power residues of 2 and of the target (times a rare prime or 3
+// more where those narrow it), and about 40 % of the
 // primes (Proth k = 3) divide no term at all.  The walk then visits only
 // n = r, r + M, r + 2M, ... with the same baby-step/giant-step blocks over
-// w(n) = 2^-n: block b's 32 terms are zeros iff its state equals one of the
-// targets wt * 2^(M j), the giant step multiplies by 2^-32M.  Every term of
+// w(n) = 2^-n, B = 32 or 64 terms each: a block's terms are zeros iff its
+// state, one term past its end, equals one of the targets wt * 2^(-M i), i = 1
+// .. B, and the giant step multiplies by 2^(-B M) (class_blocks).  Every term of
 // the class is still tested exactly, so the hits are those of the full walk.
 
 // x * w mod p for x < 2^64, w < p < 2^63, with Shoup's quotient
@@ -2342,8 +2344,8 @@ __global__ void __launch_bounds__(256, 4) classify_kernel(JobView job, const uin
 }
 
 // Tiles of 256 x REFINE_PER_THREAD listed primes per CTA, sorted by their q
-// in shared memory before the powers: the logarithm's giant steps, z^(q-8)
-// and the inverse mod q run as long as the warp's largest q, so warps of
+// in shared memory before the powers: the logarithm's giant steps and the
+// inverse mod q run as long as the warp's largest q, so warps of
 // like q keep their lanes busy (in list order 22 of 32 lanes were active).
 constexpr int REFINE_PER_THREAD = 2;
 template <uint32_t FAM, class MT>
@@ -3052,8 +3054,8 @@ int launch_batch(BatchJob *d_jobs, const uint32_t *d_active, const uint32_t gcou
 }
 
 // --------------------------------------------------------- the prime 2
-// value_mod_2 / next_value_mod_2 of each family (number_sequence_helpers.hpp:14-37
-// and the per-family closed forms cited in the oracle).
+// value_mod_2 of each family (number_sequence_helpers.hpp:14-37 and the
+// per-family closed forms cited in the oracle).
 __device__ __forceinline__ uint64_t value_mod_2(uint32_t fam, uint64_t param, uint64_t n)
 {
     switch (fam) {

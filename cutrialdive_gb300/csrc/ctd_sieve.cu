@@ -637,7 +637,7 @@ uint64_t prime_count_upper_bound(uint64_t lo, uint64_t hi)
 
 // ------------------------------------------------ launch-only variant
 // For the batched engine: base primes and window scratch are prepared once,
-// then each segment is three kernel launches with the prime count left in
+// then each segment is four kernel launches with the prime count left in
 // device memory -- no allocation and no host wait, so a whole schedule of
 // segments can be captured in one CUDA graph.
 int sieve_prepare_base(SieveWorkspace *ws, uint64_t hi, cudaStream_t st, std::string &err)
@@ -695,7 +695,7 @@ int sieve_odd_async(SieveWorkspace *ws, uint64_t lo, uint64_t hi, uint64_t *d_ou
 }
 
 // ----------------------------------------------- fixed-scratch variant
-// The same three-pass sieve over scratch the caller provides (no device
+// The same sieve, without the pass for the first multiples, over scratch the caller provides (no device
 // allocation, no cached state): base primes are recomputed on every call
 // into `sc.base`, whose unused tail is filled with 0xffffffff so the kernels'
 // "p^2 beyond the window" test stops at the real list.

@@ -110,8 +110,10 @@ typedef struct ctd_tuning {
     int32_t block_size;        /* threads per CTA: 32..256, a multiple of 32 */
     int32_t ctas_per_sm;       /* CTAs per SM of the persistent grid; 0 = as many as fit */
     uint32_t items_per_thread; /* below this many (prime, tile) items per resident thread, index ranges are tiled */
-    uint32_t min_tile;         /* shortest index tile (each tile starts with an O(log n) jump) */
-    uint32_t segment_log2;     /* default prime-segment width of ctd_run_plain, log2; 0 = 26 */
+    uint32_t min_tile;         /* shortest index tile (each tile starts with an O(log n) jump); a context without
+                                  an entry cuts shorter ones where a list would leave threads idle */
+    uint32_t segment_log2;     /* default prime-segment width of ctd_run_plain, log2; 0 = 26, or 28 without a
+                                  callback (see ctd_run_plain) */
     uint32_t variant;          /* step form, CTD_VARIANT_* (results never depend on it) */
     uint32_t classify_min;     /* Proth/Riesel/Mersenne: index ranges at least this long walk only the
                                   power-residue class of their zeros; 0 = 8192 */
@@ -179,7 +181,10 @@ int ctd_check_job(const ctd_job *job);
  * report the excess (src/factors_buffer.hpp:62-75).  Primes p <= resume_after_prime are
  * skipped (src/trial_factoring.cuh:404).  segment_length 0 = the tuned
  * length for the job's family and first prime width (untuned 2^26; 2^28
- * without a callback, where the device has the room).  Across
+ * without a callback, where the device has the room: the context then keeps
+ * its buffers for 2^28 until it is closed, 8 bytes for each prime that the
+ * range may hold and, Proth, Riesel and Mersenne over long index ranges, 61 a
+ * prime -- 0.2 and 0.7 GB at 2^33).  Across
  * the host link the call moves only what it must: an all-zero resume state
  * is cleared on the device instead of uploaded, and the counts come back
  * with the occupied slots only (the host slots past a count stay zero).
@@ -211,7 +216,11 @@ int ctd_sieve_device(ctd_ctx *ctx, uint64_t lo, uint64_t hi, uint64_t *d_out, ui
  * different streams.  The class buffers of the Proth, Riesel and Mersenne
  * launches (about 61 bytes per prime of the largest list, kept by the
  * context) are allocated on first need; where the device cannot give them,
- * the call walks every term instead, with the same results. */
+ * the call walks every term instead, with the same results.  Captured into a
+ * graph, such a call needs them allocated before, and the graph is valid until
+ * a longer list makes them grow.  Fibonacci and Lucas launches keep a list of
+ * 24 bytes for a part of the primes; into a graph they go without it.  They are
+ * fastest for lists in ascending order that hold most primes of their range. */
 int ctd_residues_device(ctd_ctx *ctx, const ctd_job *job, const uint64_t *d_primes, uint64_t nprimes,
                         uint32_t *d_counts, uint64_t *d_factors, void *stream);
 
