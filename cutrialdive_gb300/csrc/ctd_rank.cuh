@@ -720,6 +720,7 @@ static cudaError_t launch_ranks(const JobView &v, const uint64_t *d_primes, uint
     // 584,000 primes around 2^34: 4.1 ms in index tiles, 2.0 whole; 29,000 at
     // 2^33: 0.38 and 0.67.
     JobView w = v;
+    walk_block = walk_block < 256 ? walk_block : 256;
     const uint64_t threads = (uint64_t)walk_grid * walk_block;
     if (any && fibonacci_rank_pays(v.n0, v.n1) && (n >= threads || (4 * n >= threads && v.n1 >= 1u << 14))) {
         w.tiles = 1;

@@ -3383,6 +3383,10 @@ int launch_residues(const JobView &view, const uint64_t *d_primes, uint64_t npri
             return rc0;
         next = &scratch->counters->next;
     }
+    // (the tiles of ranks and orders take no launch shape, so a block size beyond
+    // the walks' 256 threads must not fail the lists that are walked instead)
+    if (block > 256 && (view.family == FIBONACCI || view.family == LUCAS || view.family == MERSENNE))
+        block = 256;
     cudaError_t rc;
     switch (view.family) {
     case MERSENNE: rc = launch_fam<MERSENNE>(view, d_primes, nprimes, grid, block, stream, next); break;

@@ -58,3 +58,47 @@ def test_lists(eng, family):
             finally:
                 eng.set_tuning(family, None)
         assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1]), primes[:3]
+
+
+@pytest.mark.parametrize("block", [64, 512])
+@pytest.mark.parametrize("family,f0", [(O.FIBONACCI, 1 << 62), (O.LUCAS, (1 << 62) - (1 << 15)), (O.MERSENNE, 1 << 62),
+                                       (O.MERSENNE, (1 << 62) - (1 << 15))])
+def test_launch_shapes(family, f0, block):
+    """A launch shape has no effect on tiles of ranks; where a range around 2^62 is
+    walked instead, one beyond the walk's 256 threads is not an error either."""
+    eng = ctd.Engine(0)
+    try:
+        out = []
+        for shape in (0, block):
+            eng.set_launch(0, shape)
+            buf = ctd.factors_buffer.empty(1, TERMS, 32)
+            eng.run_plain(ctd.CtdJob(family, 32, 0, 1, 1 + TERMS, f0, f0 + (1 << 16)), buf)
+            out.append(str(buf.to_factoring_results()))
+        assert out[0] == out[1]
+    finally:
+        eng.close()
+
+
+@pytest.mark.parametrize("block", [64, 512])
+@pytest.mark.parametrize("family", [O.FIBONACCI, O.LUCAS])
+def test_launch_shapes_of_lists(family, block):
+    torch = pytest.importorskip("torch")
+    eng = ctd.Engine(0)
+    L = ctd.load_native()
+    try:
+        primes = mixed(eng, 0.5)
+        job = ctd.CtdJob(family, 32, 0, 1, 1 + TERMS, int(primes.min()), int(primes.max()) + 1)
+        d = torch.from_numpy(primes.view(np.int64)).cuda()
+        out = []
+        for shape in (0, block):
+            eng.set_launch(0, shape)
+            counts = torch.zeros(TERMS, dtype=torch.int32, device="cuda")
+            factors = torch.zeros((TERMS, 32), dtype=torch.int64, device="cuda")
+            torch.cuda.synchronize()
+            assert L.ctd_residues_device(eng.handle, job, d.data_ptr(), d.numel(), counts.data_ptr(),
+                                         factors.data_ptr(), None) == 0
+            torch.cuda.synchronize()
+            out.append((counts.cpu().numpy(), np.sort(factors.cpu().numpy(), axis=1)))
+        assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    finally:
+        eng.close()
