@@ -508,7 +508,7 @@ def run_ours(args, world, rank, local):
     sieve_s = statistics.mean(sieve_ms) * 1e-3
     hbm = measured_peaks().get("hbm_gbs")
     sieve_bytes = statistics.mean(nodd) * 8
-    sieve = {"kernel": "device sieve (sieve_windows + scan_counts + compact_windows, host count readback)",
+    sieve = {"kernel": "device sieve (sieve_starts + sieve_windows + scan_counts + compact_chunks, host count readback)",
              "ms_per_step": statistics.mean(sieve_ms), "primes_per_step": statistics.mean(nodd),
              "achieved_gbs": sieve_bytes / sieve_s / 1e9, "peak_gbs": hbm,
              "frac": (sieve_bytes / sieve_s / 1e9 / hbm) if hbm else None,

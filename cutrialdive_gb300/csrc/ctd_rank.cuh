@@ -615,7 +615,7 @@ rank_walk_kernel(JobView job, const uint64_t *__restrict__ primes, uint64_t npri
         residue_items<FAM>(job, primes, nprimes, next);
 }
 
-// Bound by integer issue (56 % of the slots, 20 of 32 lanes): the powers, about
+// Bound by integer issue (61 % of the slots, 20 of 32 lanes): the powers, about
 // 20 bits of two narrow Montgomery products each, are the largest part, then
 // the marks and the primes' multiples.  A tile of 1024 primes shares one walk
 // over the 5133 primes below 50000.  The 2.8 million primes of a 2^26-wide
