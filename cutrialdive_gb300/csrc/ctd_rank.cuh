@@ -576,7 +576,9 @@ __device__ __forceinline__ bool rank_sparse(const uint32_t *sparse, uint64_t npr
     return sparse && 4ull * *sparse > (nprimes + tile - 1) / tile;
 }
 
-// a warp a tile; bound by reading the list once
+// a warp a tile; bound by the latency of reading the list once, by few warps: 31 us
+// for 5.7 million primes from DRAM, 2 % of rank_kernel's 1.2 ms for them (n = 1..50000;
+// reads unrolled by eight take as long)
 __global__ void __launch_bounds__(256) rank_fit_kernel(const uint64_t *__restrict__ primes, uint64_t nprimes,
                                                        uint32_t tile, uint32_t *sparse)
 {
